@@ -4,8 +4,8 @@
 // The candidate arithmetic (eik_eval.cuh) gives every node the smallest of
 // its seed and of the candidate times its fast-marching update events
 // produce.  The solve is a fast iterative method over a field's active list:
-// each step evaluates every listed node once (a thread per node), commits the
-// new values and lists the nodes a changed node can move.  A time window
+// each step evaluates every listed node once, commits the new values and lists
+// the nodes a changed node can move.  A time window
 // bounds what may be committed: a node whose new time lies beyond it waits
 // (it records the time and stays listed; until an input changes or the
 // window reaches that time, listing it costs a compare), and the window moves
@@ -17,11 +17,11 @@
 // One thread block owns a field for the whole solve: the lists, the
 // "listed" bitset and the window live in shared memory, steps are separated
 // by block barriers instead of kernel launches, and the field's front stays
-// in the SM's L1.  A step has four phases separated by barriers: evaluate
-// (reads committed state only, stages new values per slot), arbitrate,
-// commit, spread.  Evaluations never see a value of the same step, so the
-// result does not depend on thread timing: a forward is bit-identical run to
-// run.
+// in the SM's L1.  A step's phases are separated by barriers: evaluate the
+// regular quadrants, evaluate the cut cells (both read committed state only
+// and stage new values), arbitrate and commit, spread.  Evaluations never see
+// a value of the same step, so the result does not depend on thread timing or
+// block size: a forward is bit-identical run to run.
 //
 // Arithmetic is FP64 with the reference's expression order; this file is
 // compiled with --fmad=false so candidate times are bit-identical to the
@@ -30,7 +30,7 @@
 #include <climits>
 #include <mutex>
 #include "eik64.cuh"
-#include "eik_eval.cuh"
+#include "eik_coop.cuh"
 #include "model.h"
 
 namespace fmt2d {
@@ -46,40 +46,32 @@ using namespace ev;
 // workload (e64_solve_sizes, fmt2d_autotune).
 constexpr int kSolveSizes[3] = {256, 384, 512};
 constexpr int kSolveDefault = 384;
-constexpr unsigned kLCap = 4096;          // entries of each list held in shared memory
-constexpr unsigned kCCap = 2048;          // commit entries held in shared memory
+constexpr unsigned kLCap = 2048;          // regular nodes of each list held in shared memory
+constexpr unsigned kXCap = 512;           // nodes next to an interface, likewise
+constexpr unsigned kXBatch = 256;         // of those, evaluated between two barriers
+constexpr unsigned kCCap = 512;           // commits held in shared memory
 constexpr int kTileRows = 8;              // a tile: 8 slot rows x 32 slot columns (one bitset word per row)
 constexpr int kTilesMax = 12288;          // tiles per field (tile minima live in shared memory)
 constexpr size_t kSmemMax = 227 * 1024;   // dynamic shared memory of the solve block
 constexpr unsigned kSpreadBit = 0x80000000u;   // commit entry: the node moved
-constexpr unsigned kLostBit = 0x40000000u;     // commit entry: lost arbitration, listed again
+constexpr unsigned kCutBit = 0x40000000u;      // commit entry: next to an interface
 constexpr unsigned kSlotMask = 0x3fffffffu;
 constexpr unsigned long long kNone = ULLONG_MAX;
 
 struct SolveShared {
   Fld64 F;
-  unsigned cnt[2];                 // list lengths
-  unsigned nc[2];                  // commit list length, by step parity
-  int changed[2];                  // a committed write moved a node, by step parity
-  int cutstep[2];                  // the step evaluated a node next to an interface
+  unsigned cnt[2][2];              // list lengths: [list][regular, next to an interface]
+  unsigned nc;                     // commits
+  unsigned nw[2];                  // commits that moved a node (winners): regular, others
+  int changed[2];                  // a node moved, by step parity
+  int any[2];                      // a node was listed, by step parity
   unsigned nready[2];              // tiles to release, by release parity
+  int released[2];                 // a release listed a node, by release parity
   unsigned long long gmin[2];      // earliest waiting time (bits of a positive double)
   int err;
+  long long c0;                    // thread 0: cycles per phase
+  unsigned long long cyc[5], steps_cut;
 };
-
-__device__ __forceinline__ unsigned get_entry(const unsigned* sl, const unsigned* ov, unsigned i) {
-  return i < kLCap ? sl[i] : ov[i - kLCap];
-}
-
-// List slot s unless it is listed already (bits: one bit per slot).
-__device__ __forceinline__ void push(unsigned* bits, unsigned* sl, unsigned* ov, unsigned* cnt,
-                                     unsigned s) {
-  const unsigned bit = 1u << (s & 31);
-  if (atomicOr(bits + (s >> 5), bit) & bit) return;
-  const unsigned p = atomicAdd(cnt, 1u);
-  if (p < kLCap) sl[p] = s;
-  else ov[p - kLCap] = s;
-}
 
 __device__ __forceinline__ unsigned long long dbits(double d) {
   return (unsigned long long)__double_as_longlong(d);
@@ -89,7 +81,25 @@ __host__ __device__ inline int tiles_of(const Fld64& F) {
   return ((F.H + 2 + kTileRows - 1) / kTileRows) * (F.pitch / 32);
 }
 
+// Shared-memory plan of a solve launch.
+struct SolvePlan {
+  int bits;        // words of a bitset over the slots of the largest field
+  int nbits;       // bitsets in shared memory: 1 listed, 2 and waiting
+  int tiles;       // tiles of the largest field if a field has a window, else 0
+  int mwords;      // moving bitmap: words per row (a power of two), and in all
+  int mtotal;
+};
+
 // Solve every field of the batch from its list_in (one block per field).
+//
+// A list holds its regular nodes and its nodes next to an interface apart: a
+// thread evaluates one of the former or the regular quadrants of one of the
+// latter, then sixteen lanes evaluate a node's cut cells (eik_coop.cuh).
+//
+// The nodes that move in a step mark a small bitmap (all rows, columns modulo
+// 32 * mwords) and claim their new time in global memory with the step's
+// stamp; a node looks up only the claims of marked neighbours, and the stamp
+// tells a mark of another column or step.
 //
 // Waiting nodes: a node whose new time lies beyond the window records it in
 // pend and sets its bit in the waiting bitset; each tile of 8 x 32 slots
@@ -99,127 +109,264 @@ __host__ __device__ inline int tiles_of(const Fld64& F) {
 // waiting node whose input changes is listed at once (its recorded time was
 // computed from the old value).
 //
-// Shared memory: the two lists, the commit list, the tile minima and the
-// list of tiles to scan, and (when they fit) the listed and waiting bitsets;
-// smem_bits is the bitset size in words that fits, larger fields use their
-// global bitsets.
+// What bounds it: a step's chain of instructions (a warp runs each phase once
+// or twice a step, at about 8 cycles an instruction) times the steps of a
+// field.  2001x401, Pg+PmP, 30 sources: 16 us a step (51 us with a thread per
+// node and three arrays), 0.21 s a forward (0.72 s).  384 threads: 256 give
+// 0.23 s (too few warps for a front of 300 nodes), 512 give 0.26 s (128
+// registers, spills).  A cluster of blocks per field was tried and was slower
+// where it was compared, with an earlier form of the evaluation (1 source:
+// 0.18 s with 8 blocks per field against 0.15 s now with one): a cluster
+// barrier that publishes global stores takes 1600 cycles against 45 for the
+// block's own.
 template <int kSolveThreads>
 __global__ void __launch_bounds__(kSolveThreads, 1)
-    k_solve(Fld64* fields, int nf, int smem_bits, int nsmem, int tiles_cap, long long max_steps,
-            unsigned long long* ctr) {
-  constexpr int kSolveWarps = kSolveThreads / 32;
-  constexpr int kHalfWarps = kSolveThreads / 16;
+    k_solve(Fld64* fields, SolvePlan P, long long max_steps, unsigned long long* ctr) {
+  constexpr int kWarps = kSolveThreads / 32;
   extern __shared__ __align__(16) unsigned char dsm_raw[];
   __shared__ SolveShared sh;
+  __shared__ CutWork cutw[2 * kWarps];
+  // regular candidates of the nodes next to an interface, by place in the batch
+  __shared__ RegBest xrb[kXBatch];
+  __shared__ uint32_t xcode[kXBatch];
+  // commits: slot and flags, new and old time, gradient, flags; winners
+  __shared__ unsigned ce[kCCap];
+  __shared__ double cT[kCCap], co[kCCap], cgx[kCCap], cgz[kCCap];
+  __shared__ uint8_t cf[kCCap];
+  __shared__ unsigned short cw[kCCap];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int hw = tid >> 4, hl = tid & 15;                 // half-warp, its lane
-  const unsigned hmask = 0xffffu << (16 * (hw & 1));
   if (tid == 0) {
     sh.F = fields[blockIdx.x];
-    sh.cnt[0] = sh.cnt[1] = 0u;
-    sh.nc[0] = sh.nc[1] = 0u;
-    sh.changed[0] = sh.changed[1] = 0;
-    sh.cutstep[0] = sh.cutstep[1] = 0;
-    sh.nready[0] = sh.nready[1] = 0u;
-    sh.gmin[0] = sh.gmin[1] = kNone;
+    for (int k = 0; k < 2; ++k) {
+      sh.cnt[k][0] = sh.cnt[k][1] = 0u;
+      sh.changed[k] = sh.any[k] = sh.released[k] = 0;
+      sh.nready[k] = 0u;
+      sh.gmin[k] = kNone;
+    }
+    sh.nc = sh.nw[0] = sh.nw[1] = 0u;
     sh.err = 0;
+    for (int k = 0; k < 5; ++k) sh.cyc[k] = 0;
+    sh.steps_cut = 0;
   }
   __syncthreads();
   const Fld64& F = sh.F;
+  const unsigned pitch = (unsigned)F.pitch;
+  const double rdx = 1.0 / F.dx;
   const unsigned ns = (unsigned)F.nslots();
   const unsigned nbw = (ns + 31u) >> 5;
   const int tcols = F.pitch / 32, ntiles = tiles_of(F);
+  // row of a slot: s / pitch for s < 2^30 by a multiplication (the quotient is
+  // exact because the multiplier's error times 2^30 stays below one)
+  const int mshift = 30 + (32 - __clz((int)pitch - 1));
+  const unsigned long long mmul = ((1ull << mshift) + pitch - 1) / pitch;
+  auto row_of = [&](unsigned s) { return (int)(((unsigned long long)s * mmul) >> mshift); };
   unsigned long long* tmin = reinterpret_cast<unsigned long long*>(dsm_raw);
-  unsigned* sl[2];
-  sl[0] = reinterpret_cast<unsigned*>(tmin + tiles_cap);
-  sl[1] = sl[0] + kLCap;
-  unsigned* scl = sl[1] + kLCap;
-  unsigned short* ready = reinterpret_cast<unsigned short*>(scl + kCCap);
-  unsigned* sbits = reinterpret_cast<unsigned*>(ready + tiles_cap);
-  // the bitsets in shared memory, as many as fit in order of use: listed
-  // (atomics on every push), moving (read by arbitration), waiting
-  const int nloc = nbw <= (unsigned)smem_bits ? nsmem : 0;
-  unsigned* bits = nloc >= 1 ? sbits : F.inq;
-  unsigned* mbits = nloc >= 2 ? sbits + smem_bits : F.moving;
-  unsigned* wbits = nloc >= 3 ? sbits + 2 * smem_bits : F.wait;
+  unsigned* sx = reinterpret_cast<unsigned*>(tmin + P.tiles);   // [2][kXCap]
+  unsigned* sl = sx + 2 * kXCap;                                // [2][kLCap]
+  unsigned short* ready = reinterpret_cast<unsigned short*>(sl + 2 * kLCap);
+  unsigned* mbits = reinterpret_cast<unsigned*>(ready + P.tiles);
+  unsigned* sbits = mbits + P.mtotal;
+  unsigned* bits = P.nbits >= 1 ? sbits : F.inq;
+  unsigned* wbits = P.nbits >= 2 ? sbits + P.bits : F.wait;
+  const unsigned mmask = (unsigned)P.mwords - 1u;
+  // lists: regular nodes overflow to the front of the list's part of over,
+  // the others to its back (together at most the field's slots)
+  unsigned* cov = F.over + 2 * (size_t)ns;
   // a field without a window never holds a node back: nothing waits
   const bool windowed = F.clock[1] < kReachD;
-  unsigned* ov[2] = {F.over, F.over + ns};
-  unsigned* cov = F.over + 2 * (size_t)ns;
+  // The collective steps below are called by whole warps: places in a list or
+  // the commits for the lanes that want one (one atomic per warp).
+  auto place = [&](unsigned* n, bool want) -> unsigned {
+    const unsigned m = __ballot_sync(kFull, want);
+    if (!m) return 0u;
+    unsigned p = 0;
+    const int first = __ffs(m) - 1;
+    if (lane == first) p = atomicAdd(n, (unsigned)__popc(m));
+    return __shfl_sync(kFull, p, first) + __popc(m & ((1u << lane) - 1u));
+  };
+  auto put = [&](int l, bool regular, unsigned s, unsigned p) {
+    if (regular) {
+      if (p < kLCap) sl[l * kLCap + p] = s;
+      else F.over[l * (size_t)ns + (p - kLCap)] = s;
+    } else {
+      if (p < kXCap) sx[l * kXCap + p] = s;
+      else F.over[l * (size_t)ns + (ns - 1 - (p - kXCap))] = s;
+    }
+  };
+  // List the wanting lanes' slots s in list l unless they are listed already.
+  auto push = [&](int l, unsigned s, bool regular, bool want) {
+    if (want) {
+      const unsigned bit = 1u << (s & 31);
+      want = !(atomicOr(bits + (s >> 5), bit) & bit);
+    }
+    const unsigned p = place(&sh.cnt[l][0], want && regular);
+    if (want && regular) put(l, true, s, p);
+    const unsigned x = place(&sh.cnt[l][1], want && !regular);
+    if (want && !regular) put(l, false, s, x);
+  };
+  constexpr uint32_t kPlain = kInRegion | kUpdatable | kFullyRegular;
+  auto plain = [&](unsigned s) { return (FMT_RO(F.code + s) & kPlain) == kPlain; };
+  auto waits = [&](unsigned w) { return P.nbits >= 2 ? wbits[w] : __ldcg(wbits + w); };
+  auto xentry = [&](int l, unsigned i) {
+    return i < kXCap ? sx[l * kXCap + i] : F.over[l * (size_t)ns + (ns - 1 - (i - kXCap))];
+  };
   for (unsigned w = tid; w < nbw; w += kSolveThreads) {
     bits[w] = 0u;
-    wbits[w] = 0u;
-    mbits[w] = 0u;
+    if (windowed) wbits[w] = 0u;
   }
-  for (int t = tid; t < ntiles; t += kSolveThreads) tmin[t] = kNone;
+  for (int w = tid; w < P.mtotal; w += kSolveThreads) mbits[w] = 0u;
+  if (windowed)
+    for (int t = tid; t < ntiles; t += kSolveThreads) tmin[t] = kNone;
   __syncthreads();
-  {
-    const unsigned n0 = F.cnt[0];
-    for (unsigned i = tid; i < n0; i += kSolveThreads)
-      push(bits, sl[0], ov[0], &sh.cnt[0], F.list_in[i]);
+  const unsigned n0 = F.cnt[0];
+  for (unsigned i = tid; i - lane < n0; i += kSolveThreads) {
+    const bool live = i < n0;
+    const unsigned s = live ? F.list_in[i] : 0u;
+    push(0, s, live && plain(s), live);
   }
-  __syncthreads();
   double W = F.clock[0];
   const double wstep = F.clock[1];
-  unsigned long long n_eval = 0, n_write = 0, n_rel = 0, n_cut = 0;
-  unsigned long long cyc[5] = {0, 0, 0, 0, 0};   // thread 0: cycles per phase
-  unsigned long long steps_cut = 0;
-  long long c0 = clock64();
+  // claims of earlier solves of this field carry smaller steps
+  const unsigned long long stamp0 = dbits(F.clock[2]) + 1;
+  // this thread's counts (a warp's sum stays below 2^32: it evaluates a node
+  // in microseconds)
+  unsigned n_eval = 0, n_write = 0, n_rel = 0, n_cut = 0;
+  __syncthreads();
+  if (tid == 0) sh.c0 = clock64();
+  auto lap = [&](int k) {   // (thread 0)
+    const long long c1 = clock64();
+    sh.cyc[k] += (unsigned long long)(c1 - sh.c0);
+    sh.c0 = c1;
+  };
   int cur = 0, rp = 0;
   long long it = 0;
-  for (;; ++it) {
-    const unsigned n = sh.cnt[cur];
-    if (n == 0u) break;
+  bool more = n0 != 0u;
+  for (; more; ++it) {
     if (it >= max_steps) {
       if (tid == 0) sh.err = 1;
       break;
     }
     const int par = (int)(it & 1), nxt = cur ^ 1;
-    // evaluate: read committed state only, stage what changes
-    for (unsigned i = tid; i < n; i += kSolveThreads) {
-      const unsigned s = get_entry(sl[cur], ov[cur], i);
-      atomicAnd(bits + (s >> 5), ~(1u << (s & 31)));
-      const uint32_t code = FMT_RO(F.code + s);
-      const NewV nv = evaluate(F, (int)s);
-      ++n_eval;
-      if (!(code & kFullyRegular)) {
-        ++n_cut;
-        sh.cutstep[par] = 1;
+    const unsigned long long stamp = stamp0 + (unsigned long long)it;
+    // evaluate: read committed state only, stage what changes (collective; on:
+    // the lane holds node s's new value)
+    auto stage = [&](bool on, unsigned s, unsigned cut, const NewV& nv, const Self& me) {
+      bool commit = false;
+      if (on) {
+        atomicAnd(bits + (s >> 5), ~(1u << (s & 31)));
+        ++n_eval;
+        if (!nv.write) {
+          if (windowed) F.pend[s] = -1.0;
+        } else if (nv.T < kReachD && nv.T > W) {   // beyond the window: wait for it
+          F.pend[s] = nv.T;
+          atomicOr(wbits + (s >> 5), 1u << (s & 31));
+          const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+          atomicMin(tmin + (row / kTileRows) * tcols + (col >> 5), dbits(nv.T));
+        } else {
+          if (windowed) F.pend[s] = -1.0;
+          commit = true;
+        }
       }
-      if (!nv.write) {
-        F.pend[s] = -1.0;
-        continue;
+      const unsigned p = place(&sh.nc, commit);
+      if (!commit) return;
+      const uint8_t fl =
+          (uint8_t)((me.fl & kFlSeed) | (nv.copy ? kFlCopy : 0) | (nv.sus ? kFlSusp : 0));
+      const unsigned e = s | cut | (nv.spread ? kSpreadBit : 0u);
+      if (p < kCCap) {
+        ce[p] = e;
+        cT[p] = nv.T;
+        co[p] = me.T;
+        cgx[p] = nv.gx;
+        cgz[p] = nv.gz;
+        cf[p] = fl;
+      } else {
+        cov[p - kCCap] = e;
+        F.Tn[s] = nv.T;
+        F.Gn[s] = make_double2(nv.gx, nv.gz);
+        F.fln[s] = fl;
       }
-      if (nv.T < kReachD && nv.T > W) {   // beyond the window: wait for it
-        F.pend[s] = nv.T;
-        atomicOr(wbits + (s >> 5), 1u << (s & 31));
-        const int row = (int)(s / (unsigned)F.pitch), col = (int)(s - (unsigned)row * F.pitch);
-        atomicMin(tmin + (row / kTileRows) * tcols + (col >> 5), dbits(nv.T));
-        continue;
-      }
-      F.pend[s] = -1.0;
-      F.Tn[s] = nv.T;
-      F.Gn[s] = make_double2(nv.gx, nv.gz);
-      F.fln[s] = (uint8_t)((F.fl[s] & kFlSeed) | (nv.copy ? kFlCopy : 0) | (nv.sus ? kFlSusp : 0));
-      const unsigned p = atomicAdd(&sh.nc[par], 1u);
-      const unsigned e = s | (nv.spread ? kSpreadBit : 0u);
-      if (p < kCCap) scl[p] = e;
-      else cov[p - kCCap] = e;
       if (nv.spread) {
         sh.changed[par] = 1;
-        F.claim[s] = dbits(nv.T);
-        atomicOr(mbits + (s >> 5), 1u << (s & 31));
+        F.claim[s] = make_ulonglong2(dbits(nv.T), stamp);
+        const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+        atomicOr(mbits + (unsigned)row * P.mwords + ((col >> 5) & mmask), 1u << (col & 31));
       }
+    };
+    const unsigned nr = sh.cnt[cur][0], nx = sh.cnt[cur][1];
+    for (unsigned x0 = 0;; x0 += kXBatch) {
+      // (the nodes next to an interface first, in warps of their own)
+      const unsigned xn = min(nx - x0, kXBatch), xpad = (xn + 31u) & ~31u;
+      const unsigned n = xpad + (x0 == 0 ? nr : 0u);
+      for (unsigned i = tid; i - lane < n; i += kSolveThreads) {
+        const bool cut = i < xpad;          // (the same in a whole warp)
+        const bool live = cut ? i < xn : i < n;
+        const unsigned k = live ? (cut ? x0 + i : i - xpad) : 0u;
+        const unsigned s = cut ? xentry(cur, k)
+                               : k < kLCap ? sl[cur * kLCap + k] : F.over[cur * (size_t)ns + (k - kLCap)];
+        const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+        const Rec me = load_rec(F, (int)s);
+        uint32_t code = kPlain;
+        unsigned act = 15u;
+        uint8_t fl = 0;
+        if (cut) {
+          code = FMT_RO(F.code + s);
+          // a node that is not updated has nothing to evaluate
+          if (!(code & kInRegion) || !(code & kUpdatable) || (int)s == F.frozen_slot) code = 0u;
+          // cells (R,D) (R,U) (L,D) (L,U) to quadrants (L,U) (R,U) (L,D) (R,D)
+          const unsigned q = row < F.H ? (code >> 4) & ~(code >> 8) & 15u : 0u;
+          act = (q >> 3) | (q & 6u) | ((q & 1u) << 3);
+        } else {
+          fl = F.fl[s];
+          if ((int)s == F.frozen_slot) act = 0u;
+        }
+        RegBest rb;
+        rb.t = rb.trig = kHugeD;
+        rb.gx = rb.gz = 0.0;
+        rb.key = kNoKey;
+        if (cut) {
+          if (act && live) rb = reg_best<true>(F, rdx, (int)s, row, col, fabs(me.v), act);
+          if (live) {
+            xrb[i] = rb;
+            xcode[i] = code;
+          }
+        } else {
+          Self self;
+          self.T = me.T;
+          self.g = make_double2(me.gx, me.gz);
+          self.fl = fl;
+          NewV nv;
+          nv.write = nv.spread = false;
+          if (act && live) {
+            rb = reg_best<false>(F, rdx, (int)s, row, col, fabs(me.v), act);
+            nv = settle(F, (int)s, rb.t, rb.gx, rb.gz, false, rb.key != kNoKey && !(rb.key & 1),
+                        rb.t, self);
+          }
+          stage(live, s, 0u, nv, self);
+        }
+      }
+      __syncthreads();
+      for (unsigned b = 2u * warp; b < xn; b += 2u * kWarps) {
+        const unsigned i = b + (lane >> 4), ii = i < xn ? i : b;
+        const unsigned s = xentry(cur, x0 + ii);
+        const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+        bool mine;
+        Self me;
+        const NewV nv = cut_best(F, cutw[2 * warp + (lane >> 4)], (int)s, row, col, xcode[ii],
+                                 xrb[ii], lane, mine, me);
+        const bool on = mine && i < xn;
+        n_cut += on;
+        stage(on, s, kCutBit, nv, me);
+      }
+      __syncthreads();
+      if (x0 + kXBatch >= nx) break;
     }
-    __syncthreads();
     if (tid == 0) {
-      const long long c1 = clock64();
-      cyc[0] += (unsigned long long)(c1 - c0);
-      if (sh.cutstep[par]) {
-        cyc[2] += (unsigned long long)(c1 - c0);
-        ++steps_cut;
+      const unsigned long long e0 = sh.cyc[0];
+      lap(0);
+      if (nx) {
+        sh.cyc[2] += sh.cyc[0] - e0;
+        ++sh.steps_cut;
       }
-      c0 = c1;
     }
     // arbitrate: a moving node commits only if no node that reads it (the
     // nodes it reads are among them) moves to a smaller (time, slot) in the
@@ -227,94 +374,275 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
     // other the earlier goes first, as the heap accepts them, so a pair that
     // hands a time back and forth (a zero-increment update) cannot swap
     // values forever.
-    const unsigned nc = sh.nc[par];
+    const unsigned nc = sh.nc;
     if (tid == 0) {
-      sh.cnt[cur] = 0u;
-      sh.nc[par ^ 1] = 0u;
+      sh.cnt[cur][0] = sh.cnt[cur][1] = 0u;
       sh.changed[par ^ 1] = 0;
-      sh.cutstep[par ^ 1] = 0;
+      sh.any[par ^ 1] = 0;
     }
-    // (a half-warp per moved node, a lane per node that reads it); a winner
-    // commits at once (nothing reads committed times in this phase; the old
-    // time stays in Tn for the spread threshold)
-    for (unsigned j = hw; j < nc; j += kHalfWarps) {
-      const unsigned e = j < kCCap ? scl[j] : cov[j - kCCap];
-      const int s = (int)(e & kSlotMask);
+    // (a thread per moved node: it reads the marks around it, then the claims
+    // of the marked ones; a winner commits at once, nothing reads committed
+    // times in this phase; its old time is kept for the spread threshold)
+    for (unsigned j = tid; j - lane < nc; j += kSolveThreads) {
+      const bool in_sh = j < kCCap, live = j < nc;
+      const unsigned e = live ? (in_sh ? ce[j] : cov[j - kCCap]) : 0u;
+      const unsigned s = e & kSlotMask;
+      const double Tn = live ? (in_sh ? cT[j] : F.Tn[s]) : 0.0;
       bool lose = false;
       if (e & kSpreadBit) {
-        // only neighbours that move this step hold a claim (moving bitset)
-        const int t = neighbour_slot(F, s, hl);
-        bool l = false;
-        if (t >= 0 && ((mbits[t >> 5] >> (t & 31)) & 1u)) {
-          const unsigned long long ks = F.claim[s], kt = F.claim[t];
-          l = kt < ks || (kt == ks && t < s);
-        }
-        lose = (__ballot_sync(hmask, l) & hmask) != 0u;
-      }
-      if (hl == 0) {
-        if (lose) {
-          if (j < kCCap) scl[j] = e | kLostBit;
-          else cov[j - kCCap] = e | kLostBit;
-          push(bits, sl[nxt], ov[nxt], &sh.cnt[nxt], (unsigned)s);
+        const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+        const unsigned long long ks = dbits(Tn);
+        // marks of columns c0 .. c0 + 4 of a slot row
+        auto marks = [&](int r, unsigned which) -> unsigned long long {
+          if (r < 0 || r >= F.H + 2) return 0ull;
+          const unsigned* m = mbits + (unsigned)r * P.mwords;
+          const int c0 = col - 2, w = c0 >> 5;
+          return __funnelshift_r(m[w & mmask], m[(w + 1) & mmask], c0 & 31) & which;
+        };
+        // the marked ones: five columns each of up to seven rows ra .. ra + 4, rb, rb + 1
+        unsigned long long mask;
+        int ra, rb;
+        if (row < F.H) {
+          // second neighbours along the axes, the 3x3 block, and the interface
+          // nodes of the columns of cells on both sides
+          ra = row - 2;
+          rb = F.H;
+          mask = marks(row, 27u) << 10 | marks(row - 1, 14u) << 5 | marks(row - 2, 4u);
+          if (row + 1 < F.H) mask |= marks(row + 1, 14u) << 15;
+          if (row + 2 < F.H) mask |= marks(row + 2, 4u) << 20;
+          mask |= marks(rb, 6u) << 25 | marks(rb + 1, 6u) << 30;
         } else {
-          if (e & kSpreadBit) ++n_write;
-          const double old = F.T[s];
-          F.T[s] = F.Tn[s];
-          F.Tn[s] = old;
-          F.G[s] = F.Gn[s];
-          F.fl[s] = F.fln[s];
+          const int side = row - F.H;
+          const int izc = FMT_RO(F.izc + side * F.pitch + col);
+          ra = F.H + (side ^ 1);
+          rb = izc - F.z_lo;
+          mask = marks(ra, 4u);
+          if (izc >= 0 && rb < F.H) mask |= marks(rb, 12u) << 25;
+          if (izc >= 0 && rb + 1 < F.H) mask |= marks(rb + 1, 12u) << 30;
+        }
+        while (mask && !lose) {
+          const int b = __ffsll((long long)mask) - 1;
+          mask &= mask - 1;
+          const int i = (b * 205) >> 10, c = col - 2 + b - 5 * i;
+          if (c < 0 || c >= F.nx) continue;
+          const unsigned t = (unsigned)(i < 5 ? ra + i : rb + i - 5) * pitch + (unsigned)c;
+          const ulonglong2 k = F.claim[t];
+          lose = k.y == stamp && (k.x < ks || (k.x == ks && t < s));
         }
       }
+      if (lose) sh.any[par] = 1;
+      push(nxt, s, !(e & kCutBit), lose);
+      const bool win = live && !lose && (e & kSpreadBit);
+      const bool wreg = win && in_sh && !(e & kCutBit), wcut = win && in_sh && (e & kCutBit);
+      const unsigned w = place(&sh.nw[0], wreg), wx = place(&sh.nw[1], wcut);
+      if (live && !lose) {
+        double* const rec = reinterpret_cast<double*>(F.R + s);
+        const double old = in_sh ? co[j] : rec[0];
+        rec[0] = Tn;
+        *reinterpret_cast<double2*>(rec + 2) = in_sh ? make_double2(cgx[j], cgz[j]) : F.Gn[s];
+        F.fl[s] = in_sh ? cf[j] : F.fln[s];
+        if (win) {
+          ++n_write;
+          if (in_sh) {
+            co[j] = fmin(old, Tn);
+            cw[wreg ? w : kCCap - 1 - wx] = (unsigned short)j;
+          } else {
+            F.Tn[s] = fmin(old, Tn);
+          }
+        }
+      }
+      // (beyond shared memory the entry itself tells the winners: their only flag
+      // is kSpreadBit)
+      if (live && !in_sh) cov[j - kCCap] = lose ? s | kCutBit : e & ~kCutBit;
     }
     __syncthreads();
-    if (tid == 0) {
-      const long long c1 = clock64();
-      cyc[1] += (unsigned long long)(c1 - c0);
-      c0 = c1;
-    }
+    if (tid == 0) lap(1);
     // spread: every candidate of a node u that involves node v is at or above
     // v's time, so a change of v from a to b can only move nodes at or above
     // min(a, b); those below are not listed unless they wait with a time
-    // computed from the old value, which is dropped
-    for (unsigned j = hw; j < nc; j += kHalfWarps) {
-      const unsigned e = j < kCCap ? scl[j] : cov[j - kCCap];
-      if (!(e & kSpreadBit)) continue;
-      const int s = (int)(e & kSlotMask);
-      if (hl == 0) atomicAnd(mbits + (s >> 5), ~(1u << (s & 31)));   // readers are done
-      if (e & kLostBit) continue;
-      const int t = spread_target_at(F, s, hl);
-      if (t < 0) continue;
-      const double thr = fmin(F.Tn[s], F.T[s]);
-      // a waiting target (its bit may be stale) drops the time it waits with
-      const bool waiting = windowed && ((wbits[t >> 5] >> (t & 31)) & 1u);
-      if (waiting) F.pend[t] = -1.0;
-      if (waiting || !(F.T[t] < thr)) push(bits, sl[nxt], ov[nxt], &sh.cnt[nxt], (unsigned)t);
+    // computed from the old value, which is dropped.  A node that passes this
+    // test without reading s counts for the window (any), but is not listed:
+    // its evaluation would change nothing
+    // A regular winner is a corner of no cut cell, so only grid nodes read it:
+    // four lanes each take its neighbour along an axis, the one behind that and
+    // a diagonal one
+    const unsigned nw = sh.nw[0], nwx = sh.nw[1], no = nc > kCCap ? nc - kCCap : 0u;
+    for (unsigned k = tid; k - lane < 4u * nw; k += kSolveThreads) {
+      const bool live = (k >> 2) < nw;
+      const unsigned j = cw[live ? k >> 2 : 0u];
+      const int d = (int)(k & 3u), sgn = (d & 1) ? 1 : -1;
+      const unsigned s = ce[j] & kSlotMask;
+      const double thr = co[j];
+      const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+      const int dr = d < 2 ? 0 : sgn, dc = d < 2 ? sgn : 0;
+      // (diagonal: (-1,-1) (-1,1) (1,-1) (1,1))
+      const int rr[3] = {row + dr, row + 2 * dr, row + (d < 2 ? -1 : 1)};
+      const int cc[3] = {col + dc, col + 2 * dc, col + sgn};
+      unsigned t[3];
+      double2 tv[3];
+      bool want[3];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        want[h] = live && rr[h] >= 0 && rr[h] < F.H && cc[h] >= 0 && cc[h] < F.nx;
+        t[h] = want[h] ? (unsigned)(rr[h] * (int)pitch + cc[h]) : s;
+        tv[h] = *reinterpret_cast<const double2*>(F.R + t[h]);
+      }
+      bool any = false;
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        // (a velocity of zero: outside the region, unless the code says otherwise)
+        if (want[h] && tv[h].y == 0.0) want[h] = (FMT_RO(F.code + t[h]) & kInRegion) != 0u;
+        // a waiting target (its bit may be stale) drops the time it waits with
+        const bool waiting = want[h] && windowed && ((waits(t[h] >> 5) >> (t[h] & 31)) & 1u);
+        want[h] = want[h] && (waiting || !(tv[h].x < thr));
+        any |= want[h];
+        // of those, the nodes whose update reads s: a second neighbour only
+        // behind a reached neighbour that is not earlier than s (T2 <= T1, at
+        // its old or new time), a diagonal one only through a cut cell
+        if (h == 1) want[h] = want[h] && tv[0].x < kReachD && tv[0].x >= thr;
+        if (h == 2) want[h] = want[h] && !(tv[h].y > 0.0);
+        if (want[h] && waiting) F.pend[t[h]] = -1.0;
+        if (want[h]) {
+          const unsigned bit = 1u << (t[h] & 31);
+          want[h] = !(atomicOr(bits + (t[h] >> 5), bit) & bit);
+        }
+      }
+      if (any) sh.any[par] = 1;
+      // places for the up to three nodes of each lane
+      const unsigned below = (1u << lane) - 1u;
+      const bool plain0 = tv[0].y > 0.0, plain1 = tv[1].y > 0.0;
+      const unsigned r0 = __ballot_sync(kFull, want[0] && plain0);
+      const unsigned r1 = __ballot_sync(kFull, want[1] && plain1);
+      const unsigned x0 = __ballot_sync(kFull, want[0] && !plain0);
+      const unsigned x1 = __ballot_sync(kFull, want[1] && !plain1);
+      const unsigned x2 = __ballot_sync(kFull, want[2]);
+      unsigned base = 0;
+      if (lane == 0 && (r0 | r1)) base = atomicAdd(&sh.cnt[nxt][0], (unsigned)(__popc(r0) + __popc(r1)));
+      if (lane == 1 && (x0 | x1 | x2))
+        base = atomicAdd(&sh.cnt[nxt][1], (unsigned)(__popc(x0) + __popc(x1) + __popc(x2)));
+      const unsigned rbase = __shfl_sync(kFull, base, 0), xbase = __shfl_sync(kFull, base, 1);
+      if (want[0])
+        put(nxt, plain0, t[0], plain0 ? rbase + __popc(r0 & below) : xbase + __popc(x0 & below));
+      if (want[1])
+        put(nxt, plain1, t[1], plain1 ? rbase + __popc(r0) + __popc(r1 & below)
+                                      : xbase + __popc(x0) + __popc(x1 & below));
+      if (want[2]) put(nxt, false, t[2], xbase + __popc(x0) + __popc(x1) + __popc(x2 & below));
+    }
+    // the others and those beyond shared memory: eight lanes per winner, two of
+    // the nodes that read it each (from the last warp down: the first ones have
+    // the regular winners)
+    for (unsigned k = (kWarps - 1 - warp) * 32 + lane; k - lane < 8u * (nwx + no);
+         k += kSolveThreads) {
+      const unsigned w = k >> 3;
+      const int sub = (int)(k & 7u);
+      bool live = w < nwx + no;
+      unsigned s = 0u;
+      double thr = 0.0;
+      if (w < nwx) {
+        const unsigned j = cw[kCCap - 1 - w];
+        s = ce[j] & kSlotMask;
+        thr = co[j];
+      } else if (live) {
+        const unsigned e = cov[w - nwx];
+        live = (e & kSpreadBit) != 0u;
+        s = e & kSlotMask;
+        thr = F.Tn[s];
+      }
+      const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+      int t[2];
+      double2 tv[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // spread_target_at's nodes, its positions q
+        const int q = sub + 8 * h;
+        int r = -1, c = col;
+        if (row < F.H) {
+          if (q < 12) {
+            // rows and columns -2..2 of the second neighbours and the 3x3 block
+            r = row + (int)((0x333221112240ull >> (4 * q)) & 15) - 2;
+            c = col + (int)((0x321313214022ull >> (4 * q)) & 15) - 2;
+            if (r >= F.H) r = -1;
+          } else {
+            // the interface nodes of the cut cells it is a corner of
+            const int side = (q - 12) >> 1;
+            c = col - 1 + (q & 1);
+            if (c >= 0 && c < F.nx) {
+              const int izc = FMT_RO(F.izc + side * F.pitch + c), ar = F.z_lo + row;
+              if (izc >= 0 && (izc == ar || izc + 1 == ar)) r = F.H + side;
+            }
+          }
+        } else {
+          const int side = row - F.H;
+          if (q == 4) {
+            r = F.H + (side ^ 1);
+          } else if (q < 4) {
+            const int izc = FMT_RO(F.izc + side * F.pitch + col);
+            r = izc < 0 ? -1 : izc - F.z_lo + (q & 1);
+            c = col + (q >> 1);
+            if (r >= F.H) r = -1;
+          }
+        }
+        t[h] = live && r >= 0 && c >= 0 && c < F.nx ? r * (int)pitch + c : -1;
+        tv[h] = t[h] >= 0 ? *reinterpret_cast<const double2*>(F.R + t[h]) : make_double2(0.0, 0.0);
+      }
+      // time of the node between s and a second neighbour (sub < 4)
+      double Tw = 0.0;
+      if (row < F.H && sub < 4 && t[0] >= 0) Tw = F.R[((int)s + t[0]) / 2].x;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        bool want = t[h] >= 0;
+        // (a velocity of zero: outside the region, unless the code says otherwise)
+        if (want && tv[h].y == 0.0 && t[h] < F.H * (int)pitch)
+          want = (FMT_RO(F.code + t[h]) & kInRegion) != 0u;
+        // a waiting target (its bit may be stale) drops the time it waits with
+        const bool waiting = want && windowed && ((waits((unsigned)t[h] >> 5) >> (t[h] & 31)) & 1u);
+        want = want && (waiting || !(tv[h].x < thr));
+        if (want) sh.any[par] = 1;
+        // of those, the nodes whose update reads s: a regular node reads along
+        // the axes only, and a second neighbour only behind a reached neighbour
+        // that is not earlier than it (T2 <= T1, at s's old or new time)
+        if (row < F.H) {
+          const int q = sub + 8 * h;
+          want = want && (q < 4 ? Tw < kReachD && Tw >= thr
+                                : !((q == 4 || q == 6 || q == 9 || q == 11) && tv[h].y > 0.0));
+        }
+        if (want && waiting) F.pend[t[h]] = -1.0;
+        push(nxt, (unsigned)t[h], tv[h].y > 0.0, want);
+      }
+    }
+    // (readers are done with the marks)
+    for (unsigned j = tid; j < nc; j += kSolveThreads) {
+      const unsigned e = j < kCCap ? ce[j] : cov[j - kCCap];
+      const unsigned s = e & kSlotMask;
+      const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
+      mbits[(unsigned)row * P.mwords + ((col >> 5) & mmask)] = 0u;
     }
     __syncthreads();
     if (tid == 0) {
-      const long long c1 = clock64();
-      cyc[3] += (unsigned long long)(c1 - c0);
-      c0 = c1;
+      sh.nc = sh.nw[0] = sh.nw[1] = 0u;
+      lap(3);
     }
     // the window moves on after a step that changed nothing inside it (or
     // listed nothing); the tiles it reaches release their due nodes, and when
     // none is due it jumps to the earliest waiting time
     const bool chg = sh.changed[par] != 0;
-    if (!chg || sh.cnt[nxt] == 0u) {
-      if (!chg) W += wstep;
-      for (;;) {
+    more = sh.any[par] != 0;
+    if (!chg) W += wstep;
+    if (!chg || !more) {
+      for (; windowed;) {
         const int q = rp & 1;
         ++rp;
         for (int t = tid; t < ntiles; t += kSolveThreads)
           if (tmin[t] != kNone && __longlong_as_double((long long)tmin[t]) <= W)
             ready[atomicAdd(&sh.nready[q], 1u)] = (unsigned short)t;
         __syncthreads();
-        const unsigned nr = sh.nready[q];
+        const unsigned nready = sh.nready[q];
         if (tid == 0) {
           sh.nready[q ^ 1] = 0u;
           sh.gmin[q ^ 1] = kNone;
+          sh.released[q ^ 1] = 0;
         }
-        for (unsigned k = warp; k < nr; k += kSolveWarps) {
+        for (unsigned k = warp; k < nready; k += kWarps) {
           const int t = ready[k];
           const int r0 = (t / tcols) * kTileRows, c0 = (t % tcols) * 32;
           // lane l takes column c0 + l of the tile's rows; the rows' loads
@@ -323,7 +651,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
           double pd[kTileRows];
 #pragma unroll
           for (int rr = 0; rr < kTileRows; ++rr)
-            word[rr] = r0 + rr < F.H + 2 ? wbits[(unsigned)((r0 + rr) * F.pitch + c0) >> 5] : 0u;
+            word[rr] = r0 + rr < F.H + 2 ? waits((unsigned)((r0 + rr) * F.pitch + c0) >> 5) : 0u;
 #pragma unroll
           for (int rr = 0; rr < kTileRows; ++rr)
             pd[rr] = (word[rr] >> lane) & 1u ? F.pend[(r0 + rr) * F.pitch + c0 + lane] : 0.0;
@@ -331,18 +659,20 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
 #pragma unroll
           for (int rr = 0; rr < kTileRows; ++rr) {
             const bool set = (word[rr] >> lane) & 1u;
-            bool clear = false;
+            bool clear = false, due = false;
+            const unsigned s = (unsigned)((r0 + rr) * F.pitch + c0 + lane);
             if (set) {
               if (pd[rr] < 0.0) {
                 clear = true;                 // listed since (an input changed)
               } else if (pd[rr] <= W) {
-                clear = true;
-                push(bits, sl[nxt], ov[nxt], &sh.cnt[nxt], (unsigned)((r0 + rr) * F.pitch + c0 + lane));
+                clear = due = true;
+                sh.released[q] = 1;
                 ++n_rel;
               } else {
                 m = min(m, dbits(pd[rr]));
               }
             }
+            push(nxt, s, due && plain(s), due);
             const unsigned cm = __ballot_sync(0xffffffffu, clear);
             if (lane == 0 && cm) wbits[(unsigned)((r0 + rr) * F.pitch + c0) >> 5] = word[rr] & ~cm;
           }
@@ -351,7 +681,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
           if (lane == 0) tmin[t] = m;
         }
         __syncthreads();
-        if (sh.cnt[nxt] != 0u) break;
+        if (more || sh.released[q]) {
+          more = true;
+          break;
+        }
         // nothing due: the earliest waiting time, if any
         unsigned long long m = kNone;
         for (int t = tid; t < ntiles; t += kSolveThreads) m = min(m, tmin[t]);
@@ -361,37 +694,31 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
         if (g == kNone) break;
         W = fmax(W, __longlong_as_double((long long)g));
       }
-      if (tid == 0) {
-        const long long c1 = clock64();
-        cyc[4] += (unsigned long long)(c1 - c0);
-        c0 = c1;
-      }
+      if (tid == 0) lap(4);
     }
     cur = nxt;
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    n_eval += __shfl_xor_sync(0xffffffffu, n_eval, o);
-    n_write += __shfl_xor_sync(0xffffffffu, n_write, o);
-    n_rel += __shfl_xor_sync(0xffffffffu, n_rel, o);
-    n_cut += __shfl_xor_sync(0xffffffffu, n_cut, o);
-  }
+  n_eval = __reduce_add_sync(kFull, n_eval);
+  n_write = __reduce_add_sync(kFull, n_write);
+  n_rel = __reduce_add_sync(kFull, n_rel);
+  n_cut = __reduce_add_sync(kFull, n_cut);
   if (lane == 0 && ctr) {
-    atomicAdd(ctr + kCtrCut, n_cut);
-    atomicAdd(ctr + kCtrEval, n_eval);
-    atomicAdd(ctr + kCtrWrite, n_write);
-    atomicAdd(ctr + kCtrPass, n_rel);
+    atomicAdd(ctr + kCtrCut, (unsigned long long)n_cut);
+    atomicAdd(ctr + kCtrEval, (unsigned long long)n_eval);
+    atomicAdd(ctr + kCtrWrite, (unsigned long long)n_write);
+    atomicAdd(ctr + kCtrPass, (unsigned long long)n_rel);
   }
   __syncthreads();
   if (tid == 0) {
     F.clock[0] = W;
+    F.clock[2] = __longlong_as_double((long long)(stamp0 + (unsigned long long)it));
     F.cnt[0] = 0u;   // start list consumed; the check refills it
     F.cnt[1] = 0u;
     F.cnt[3] = (unsigned)(it < 0xffffffffll ? it : 0xffffffffll);
     if (sh.err) F.cnt[2] = 1u;
     if (ctr) {
-      for (int k = 0; k < 5; ++k) atomicAdd(ctr + kCtrCycEval + k, cyc[k]);
-      atomicAdd(ctr + kCtrStepsCut, steps_cut);
+      for (int k = 0; k < 5; ++k) atomicAdd(ctr + kCtrCycEval + k, sh.cyc[k]);
+      atomicAdd(ctr + kCtrStepsCut, sh.steps_cut);
       atomicAdd(ctr + kCtrSteps, (unsigned long long)it);
       atomicMax(ctr + kCtrMaxSteps, (unsigned long long)it);
     }
@@ -436,6 +763,30 @@ __global__ void k_queue_seeds(Fld64* fields, int nf) {
   }
 }
 
+// Solver records of a field from its state, and the state from the records.
+__global__ void k_pack(Fld64* fields, int nf) {
+  const Fld64& F = fields[blockIdx.y];
+  const int ns = F.nslots();
+  constexpr uint32_t kPlain = kInRegion | kUpdatable | kFullyRegular;
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
+    const uint32_t code = F.code[s];
+    const double v = F.vel[s];
+    const double2 g = F.G[s];
+    F.R[s] = make_double4(
+        F.T[s], !(code & kInRegion) ? 0.0 : (code & kPlain) == kPlain ? v : -v, g.x, g.y);
+  }
+}
+
+__global__ void k_unpack(Fld64* fields, int nf) {
+  const Fld64& F = fields[blockIdx.y];
+  const int ns = F.nslots();
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
+    const double4 r = F.R[s];
+    F.T[s] = r.x;
+    F.G[s] = make_double2(r.z, r.w);
+  }
+}
+
 // ---------------------------------------------------------------- seeding
 __global__ void k_fill(Fld64* fields, int nf) {
   Fld64& F = fields[blockIdx.y];
@@ -448,9 +799,12 @@ __global__ void k_fill(Fld64* fields, int nf) {
     F.seed[i] = make_double4(kHugeD, 0.0, 0.0, 0.0);
     F.fl[i] = 0;
     F.pend[i] = -1.0;
-    F.claim[i] = ULLONG_MAX;
+    F.claim[i] = make_ulonglong2(0, 0);   // of no step
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) F.frozen_slot = -1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    F.frozen_slot = -1;
+    F.clock[2] = 0.0;
+  }
 }
 
 __device__ void put_seed(Fld64& F, int s, double t, double gx, double gz) {
@@ -691,57 +1045,68 @@ void e64_start(Fld64* f, int nf, size_t max_slots, const double* step, cudaStrea
   k_queue_seeds<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
   k_clock<<<nf, 256, 0, st>>>(f, nf, step);
 }
-// Dynamic shared memory of k_solve for a batch whose largest field has
-// max_slots slots and max_tiles tiles (tiles_cap rounded up to a multiple of
-// 8); smem_bits: words of each bitset kept in shared memory, nsmem: how many
-// of the three bitsets (listed, moving, waiting, in that order) fit there
-// (0: all in global memory).
-static size_t solve_smem(size_t max_slots, int max_tiles, int* smem_bits, int* nsmem,
-                         int* tiles_cap) {
-  const int cap = (max_tiles + 7) / 8 * 8;
-  const size_t fixed = (size_t)cap * sizeof(unsigned long long) +
-                       (2 * (size_t)kLCap + kCCap) * sizeof(unsigned) +
-                       (size_t)cap * sizeof(unsigned short);
-  const size_t nbw = (max_slots + 31) / 32;
-  const size_t room = fixed + 1024 < kSmemMax ? (kSmemMax - fixed - 1024) / sizeof(unsigned) : 0;
-  const int n = nbw == 0 ? 0 : (int)std::min<size_t>(3, room / nbw);
-  *smem_bits = n > 0 ? (int)nbw : 0;
-  *nsmem = n;
-  *tiles_cap = cap;
-  return fixed + (size_t)n * nbw * sizeof(unsigned);
-}
 int e64_tiles(const Fld64& f) { return tiles_of(f); }
 int e64_tiles_max() { return kTilesMax; }
-// k_solve may use up to kSmemMax of dynamic shared memory.  The attribute is
-// set once per device and instantiation: changing a kernel's attributes while
-// it runs (a solve of another stage chain on another stream) waits for that
-// kernel to finish, which would serialise the chains.
+
+// Dynamic shared memory of k_solve under plan P.
+static size_t solve_smem(const SolvePlan& P) {
+  return (size_t)P.tiles * (sizeof(unsigned long long) + sizeof(unsigned short)) +
+         2 * (kXCap + kLCap) * sizeof(unsigned) +
+         ((size_t)P.mtotal + (size_t)P.nbits * P.bits) * sizeof(unsigned);
+}
+
+// Largest dynamic shared memory of an instantiation; its attribute is set
+// once per device: changing a kernel's attributes while it runs (a solve of
+// another stage chain on another stream) waits for that kernel to finish,
+// which would serialise the chains.
 template <int NT>
-static void solve_attr_once() {
+static size_t solve_room() {
   static std::mutex mu;
-  static bool done[64] = {};
+  static int room[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return;
+  if (dev < 0 || dev >= 64) return 0;
   std::lock_guard<std::mutex> lock(mu);
-  if (done[dev]) return;
+  if (room[dev]) return (size_t)room[dev];
   // the opt-in limit covers static and dynamic shared memory together
   int optin = 0;
   cudaFuncAttributes fa;
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
       cudaFuncGetAttributes(&fa, k_solve<NT>) != cudaSuccess)
-    return;
+    return 0;
   const int dyn = std::min<int>((int)kSmemMax, optin - (int)fa.sharedSizeBytes);
   if (cudaFuncSetAttribute(k_solve<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) ==
       cudaSuccess)
-    done[dev] = true;
+    room[dev] = dyn;
+  return (size_t)room[dev];
 }
 
 template <int NT>
-static void solve_launch(Fld64* f, int nf, int smem_bits, int nsmem, int cap, size_t bytes,
-                         long long max_steps, unsigned long long* ctr, cudaStream_t st) {
-  solve_attr_once<NT>();
-  k_solve<NT><<<nf, NT, bytes, st>>>(f, nf, smem_bits, nsmem, cap, max_steps, ctr);
+static void solve_launch(Fld64* f, const Fld64* fh, int nf, bool windowed, long long max_steps,
+                         unsigned long long* ctr, cudaStream_t st) {
+  int rows = 0, tiles = 0, slots = 0;
+  for (int i = 0; i < nf; ++i) {
+    rows = std::max(rows, fh[i].H + 2);
+    tiles = std::max(tiles, tiles_of(fh[i]));
+    slots = std::max(slots, fh[i].nslots());
+  }
+  SolvePlan P;
+  P.bits = (slots + 31) / 32;
+  P.tiles = windowed ? (tiles + 7) / 8 * 8 : 0;
+  // what fits of: the listed bitset (an atomic on every push), the waiting
+  // bitset; the moving bitmap needs a word per row at least and takes up to
+  // eight (256 columns: marks of other columns are then rare)
+  const size_t room = solve_room<NT>();
+  P.nbits = windowed ? 2 : 1;
+  for (;; --P.nbits) {
+    for (P.mwords = 8; P.mwords > 1; P.mwords /= 2) {
+      P.mtotal = rows * P.mwords;
+      if (solve_smem(P) <= room) break;
+    }
+    P.mtotal = rows * P.mwords;
+    if (P.nbits == 0 || solve_smem(P) <= room) break;
+  }
+  k_solve<NT><<<nf, NT, solve_smem(P), st>>>(f, P, max_steps, ctr);
 }
 
 const int* e64_solve_sizes(int* n) {
@@ -749,16 +1114,18 @@ const int* e64_solve_sizes(int* n) {
   return kSolveSizes;
 }
 
-void e64_solve(Fld64* f, int nf, size_t max_slots, int max_tiles, long long max_steps,
-               unsigned long long* ctr, int threads, cudaStream_t st) {
-  int smem_bits = 0, nsmem = 0, cap = 0;
-  const size_t bytes = solve_smem(max_slots, max_tiles, &smem_bits, &nsmem, &cap);
-  if (threads == 256)
-    solve_launch<256>(f, nf, smem_bits, nsmem, cap, bytes, max_steps, ctr, st);
-  else if (threads == 512)
-    solve_launch<512>(f, nf, smem_bits, nsmem, cap, bytes, max_steps, ctr, st);
-  else
-    solve_launch<kSolveDefault>(f, nf, smem_bits, nsmem, cap, bytes, max_steps, ctr, st);
+void e64_pack(Fld64* f, int nf, size_t max_slots, cudaStream_t st) {
+  const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 1024);
+  k_pack<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
+}
+
+void e64_solve(Fld64* f, const Fld64* fh, int nf, size_t max_slots, bool windowed,
+               long long max_steps, unsigned long long* ctr, int threads, cudaStream_t st) {
+  if (threads == 256) solve_launch<256>(f, fh, nf, windowed, max_steps, ctr, st);
+  else if (threads == 512) solve_launch<512>(f, fh, nf, windowed, max_steps, ctr, st);
+  else solve_launch<kSolveDefault>(f, fh, nf, windowed, max_steps, ctr, st);
+  const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 1024);
+  k_unpack<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
 }
 void e64_verify(Fld64* f, int nf, size_t max_slots, cudaStream_t st) {
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 512);

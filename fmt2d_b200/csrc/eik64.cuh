@@ -32,19 +32,19 @@ struct Fld64 {
   double2* Gout = nullptr;          // per slot: final gradient (suspect nodes refitted)
   uint8_t* fl = nullptr;            // per slot: kFlSeed | kFlCopy | kFlSusp
   double4* seed = nullptr;          // per slot: seeded (T, gx, gz, -)
-  double* clock = nullptr;          // [0] window end, [1] window step
+  double* clock = nullptr;          // [0] window end, [1] window step, [2] steps solved so far (bits)
   int frozen_slot = -1;             // node fixed at the source (never a trigger)
   // solver scratch (per slot unless stated)
-  double* Tn = nullptr;             // new time staged by the evaluation phase
-  double2* Gn = nullptr;            // new gradient staged
-  uint8_t* fln = nullptr;           // new flags staged
+  double4* R = nullptr;             // solver record: time, velocity, gradient (k_pack)
+  double* Tn = nullptr;             // new time staged by the evaluation phase (commits beyond
+  double2* Gn = nullptr;            // those in shared memory), new gradient, new flags
+  uint8_t* fln = nullptr;
   double* pend = nullptr;           // time a deferred node waits with (< 0: none)
-  unsigned long long* claim = nullptr;   // bits of the new time of a node moving this step
+  ulonglong2* claim = nullptr;      // of a node that moves: bits of its new time, the step
   unsigned* list_in = nullptr;      // nodes to start from (seeds, re-listed nodes)
-  unsigned* over = nullptr;         // 3*nslots: list overflow (two lists) and commit overflow
+  unsigned* over = nullptr;         // 3*nslots: overflow of the two lists and of the commits
   unsigned* inq = nullptr;          // bitset over slots: listed (when not in shared memory)
   unsigned* wait = nullptr;         // bitset over slots: waiting (when not in shared memory)
-  unsigned* moving = nullptr;       // bitset over slots: moving this step (when not in shared memory)
   unsigned* cnt = nullptr;          // [0] list_in length, [1] unsettled nodes found by a check,
                                     // [2] error (1: step cap), [3] steps of the last solve
 #if defined(__CUDACC__)
@@ -92,13 +92,17 @@ void e64_init_source(Fld64* f, const double* sx, const double* sz, int nf, cudaS
 void e64_seed_iface(Fld64* f, const Seed64* d, int nd, int nx, cudaStream_t st);
 // List every seeded node and its neighbours in list_in; set the windows.
 void e64_start(Fld64* f, int nf, size_t max_slots, const double* step, cudaStream_t st);
+// Fill the solver records of the batch from T, G, vel and code.
+void e64_pack(Fld64* f, int nf, size_t max_slots, cudaStream_t st);
 // Solve every field of the batch from its list_in (one thread block per
-// field, all steps in one launch; max_tiles: the most tiles of a field,
-// e64_tiles).  max_steps bounds the steps of a field;
-// a field that reaches it sets cnt[2] = 1.
+// field, all steps in one launch).  f_host: the same descriptors in host
+// memory; windowed: some field of the batch has a time window.  max_steps
+// bounds the steps of a field; a field that reaches it sets cnt[2] = 1.
 // threads: the solve block's size, one of e64_solve_sizes (others: the
 // default); the result does not depend on it.
-void e64_solve(Fld64* f, int nf, size_t max_slots, int max_tiles, long long max_steps,
+// Afterwards T and G hold the solved times and gradients.
+void e64_solve(Fld64* f, const Fld64* f_host, int nf, size_t max_slots, bool windowed,
+               long long max_steps,
                unsigned long long* ctr, int threads, cudaStream_t st);
 const int* e64_solve_sizes(int* n);
 // Tiles of a field's waiting-node index, and the most a field may have.

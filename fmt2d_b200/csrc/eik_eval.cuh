@@ -523,7 +523,9 @@ struct NewV {
 // Keeping the seed leaves NaN on the grid node; over PmP picks of twelve test
 // models this agreed with the reference's valid flags on 96.6% of picks,
 // against 95.2% for letting a finite copy win.
-FMT_HD NewV finish(const Fld64& F, int s, const Cand& w, bool sus, double sus_t) {
+// fl, curT and cg: the node's flags, time and gradient as they stand.
+FMT_HD NewV finish(const Fld64& F, int s, const Cand& w, bool sus, double sus_t, uint8_t fl,
+                   double curT, double2 cg) {
   NewV o;
   o.write = false;
   o.spread = false;
@@ -531,7 +533,6 @@ FMT_HD NewV finish(const Fld64& F, int s, const Cand& w, bool sus, double sus_t)
   grad_of(w, gx, gz);
   double T = w.t < kReachD ? w.t : kHugeD;
   bool su = sus, cp = w.copy;
-  const uint8_t fl = ldF(F, s);
   if (fl & kFlSeed) {
     const double4 sd = F.seed[s];
     if (sd.x < kReachD) {
@@ -542,14 +543,12 @@ FMT_HD NewV finish(const Fld64& F, int s, const Cand& w, bool sus, double sus_t)
       }
     }
   }
-  const double curT = ldT(F, s);
   if (T >= kReachD) {
     T = kHugeD; gx = 0.0; gz = 0.0; su = false; cp = false;
     if (curT >= kReachD) return o;
   }
   // compared bit for bit: a NaN gradient (a seed at zero distance) must not
   // count as a change on every evaluation
-  const double2 cg = ldG(F, s);
   auto same = [](double a, double b) { return bits_of(a) == bits_of(b); };
   const bool gchg = !same(T, curT) || !same(gx, cg.x) || !same(gz, cg.y) ||
                     cp != ((fl & kFlCopy) != 0);
@@ -563,6 +562,10 @@ FMT_HD NewV finish(const Fld64& F, int s, const Cand& w, bool sus, double sus_t)
       fabs(T - curT) <= F.eps && fabs(gx - cg.x) <= F.eps && fabs(gz - cg.y) <= F.eps)
     o.spread = false;
   return o;
+}
+
+FMT_HD inline NewV finish(const Fld64& F, int s, const Cand& w, bool sus, double sus_t) {
+  return finish(F, s, w, sus, sus_t, ldF(F, s), ldT(F, s), ldG(F, s));
 }
 
 // Members of connected cut cell q of grid node (r, c), in the reference's

@@ -387,38 +387,37 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
   // solver scratch of the batch, per slot: staged time, gradient and flags,
   // pending time, start list, list and commit overflow, listed bitset
   const size_t words = (total + 31 * (size_t)nf + 31) / 32 + (size_t)nf;
-  L.sTn.alloc(total * sizeof(double));
-  L.sGn.alloc(total * sizeof(double2));
+  L.sR.alloc(total * sizeof(double4));
   L.sfln.alloc(total);
   L.spend.alloc(total * sizeof(double));
-  L.sclaim.alloc(total * sizeof(unsigned long long));
+  L.sclaim.alloc(total * sizeof(ulonglong2));
   L.slist.alloc(total * sizeof(unsigned));
   L.sover.alloc(3 * total * sizeof(unsigned));
-  L.sinq.alloc(3 * words * sizeof(unsigned));
+  L.sinq.alloc(2 * words * sizeof(unsigned));
   L.scnt.alloc((size_t)nf * 4 * sizeof(unsigned));
   L.ctr.alloc(kCtrN * sizeof(unsigned long long));
-  if (!L.sTn.p || !L.sGn.p || !L.sfln.p || !L.spend.p || !L.sclaim.p || !L.slist.p ||
+  if (!L.sR.p || !L.sfln.p || !L.spend.p || !L.sclaim.p || !L.slist.p ||
       !L.sover.p ||
       !L.sinq.p || !L.scnt.p || !L.ctr.p)
     return "device allocation failed for the solver scratch";
   size_t base = 0, wbase = 0;
-  int max_tiles = 0;
+  bool windowed = false;
   for (int i = 0; i < nf; ++i) {
     const int s = items[i].first, tf = items[i].second;
     const DevRegionStore& D = reg_[kTf[tf].reg];
     hf[i] = field_view(s, tf);
-    hf[i].Tn = L.sTn.as<double>() + base;
-    hf[i].Gn = L.sGn.as<double2>() + base;
+    hf[i].R = L.sR.as<double4>() + base;
+    // the state is in the records while a solve runs: its staging takes T and G
+    hf[i].Tn = hf[i].T;
+    hf[i].Gn = hf[i].G;
     hf[i].fln = L.sfln.as<uint8_t>() + base;
     hf[i].pend = L.spend.as<double>() + base;
-    hf[i].claim = L.sclaim.as<unsigned long long>() + base;
+    hf[i].claim = L.sclaim.as<ulonglong2>() + base;
     hf[i].list_in = L.slist.as<unsigned>() + base;
     hf[i].over = L.sover.as<unsigned>() + 3 * base;
     hf[i].inq = L.sinq.as<unsigned>() + wbase;
     hf[i].wait = L.sinq.as<unsigned>() + words + wbase;
-    hf[i].moving = L.sinq.as<unsigned>() + 2 * words + wbase;
     if (e64_tiles(hf[i]) > e64_tiles_max()) return "region too large for the eikonal solver";
-    max_tiles = std::max(max_tiles, e64_tiles(hf[i]));
     hf[i].cnt = L.scnt.as<unsigned>() + 4 * (size_t)i;
     base += D.nslots;
     wbase += (D.nslots + 31) / 32;
@@ -430,6 +429,7 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
     const double wc = window_cells > 0.0 ? window_cells
                       : (kTf[tf].level == 0 ? 0.0 : iface_window_cells);
     wstep[i] = wc > 0.0 ? wc * m_.dx / D.vmax : kHugeD;
+    windowed = windowed || wstep[i] < kReachD;
     if (tf == 5) hw.push_back(i);
   }
   std::string e;
@@ -479,7 +479,8 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
     ++L.stats.launches;
   }
   e64_start(dF, nf, max_slots, L.step.as<double>(), L.st);
-  L.stats.launches += 2;
+  e64_pack(dF, nf, max_slots, L.st);
+  L.stats.launches += 3;
   CK(cudaGetLastError());
   // solve, then check every node; nodes the check re-lists are solved again
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -496,8 +497,8 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
   cudaEventRecord(e0, L.st);
   unsigned long long bad = 0;
   for (int pass = 0;; ++pass) {
-    e64_solve(dF, nf, max_slots, max_tiles, max_steps, dctr, solve_threads, L.st);
-    ++L.stats.launches;
+    e64_solve(dF, hf.data(), nf, max_slots, windowed, max_steps, dctr, solve_threads, L.st);
+    L.stats.launches += 2;
     ++L.stats.final_passes;
     cudaMemsetAsync(L.sinq.p, 0, words * sizeof(unsigned), L.st);
     e64_verify(dF, nf, max_slots, L.st);

@@ -90,7 +90,7 @@ struct SolveLane {
   cudaStream_t st = nullptr;
   cudaEvent_t done = nullptr;
   DevBuf fields, up, step, sx, sz, seeds, which, hw, hwpre, ctr;
-  DevBuf sTn, sGn, sfln, spend, sclaim, slist, sover, sinq, scnt;
+  DevBuf sR, sfln, spend, sclaim, slist, sover, sinq, scnt;
   SolveStats stats;
   bool not_converged = false;
   // pinned staging of the lane's small host <-> device copies (descriptors,
@@ -100,7 +100,7 @@ struct SolveLane {
   char* pin = nullptr;
   size_t pin_cap = 0, pin_used = 0;
   void free_all() {
-    for (DevBuf* b : {&fields, &up, &step, &sx, &sz, &seeds, &which, &hw, &hwpre, &ctr, &sTn, &sGn, &sfln,
+    for (DevBuf* b : {&fields, &up, &step, &sx, &sz, &seeds, &which, &hw, &hwpre, &ctr, &sR, &sfln,
                       &spend, &sclaim, &slist, &sover, &sinq, &scnt})
       b->free_();
     if (pin) cudaFreeHost(pin);
