@@ -1320,7 +1320,7 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
         if (!(e = adj_put(d_dptr, dptr, stream_)).empty()) return e;
         if (!(e = adj_put(d_tp, tp, stream_)).empty()) return e;
         if (!(e = adj_put(d_tpk, tpk, stream_)).empty()) return e;
-        tr_adj_picks(d_trmodel_.as<TrModel>(), d_trfields_.as<TrField>(), d_picks_.as<TrPick>(),
+        tr_adj_picks(trmodel_, d_trfields_.as<TrField>(), d_picks_.as<TrPick>(),
                      d_entry_.as<double>(), d_coef.as<double>(), d_tgt.as<int>(), d_tp.as<int>(),
                      d_tpk.as<int>(), d_dptr.as<double* const>(), (int)tgt.size(), stream_);
         ACK(cudaGetLastError());

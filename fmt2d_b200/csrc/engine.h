@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 #include "eik64.cuh"
+#include "rays.cuh"
 #include "model.h"
 
 namespace fmt2d {
@@ -188,10 +189,11 @@ class Engine {
   long long adj_map_version_[7] = {-1, -1, -1, -1, -1, -1, -1};
   std::vector<std::array<FieldStore, 13>> fields_;
   std::vector<double> src_x_, src_z_;
+  TrModel trmodel_;           // the model as the ray kernels take it
   DevBuf export_;             // region-order copy of a field being read back
   SolveLane lanes_[kChains];
   cudaEvent_t ev_start_ = nullptr;
-  DevBuf d_pvel_, d_invidx_, d_xpos_, d_trmodel_, d_picks_, d_trfields_, d_srcx_, d_srcz_,
+  DevBuf d_pvel_, d_invidx_, d_xpos_, d_picks_, d_trfields_, d_srcx_, d_srcz_,
       d_tcalc_, d_valid_, d_cnt_, d_off_, d_rowptr_, d_tmp_, d_col_, d_val_, d_sft_, d_sfjobs_,
       d_entry_;
   int npick_ = -1, rows_ = 0;

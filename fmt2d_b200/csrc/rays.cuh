@@ -18,6 +18,8 @@ struct TrRegion {
 struct TrModel {
   int nx = 0, nz = 0;
   double x0 = 0, dx = 0, tol = 0, vwater = 1.5;
+  double xp0 = 0, vdx = 0;            // xpos[0], xpos[1] - xpos[0]
+  double rdx = 0, rvdx = 0, rvwater = 0;   // correctly rounded reciprocals of dx, vdx, vwater
   const double* vel = nullptr;        // propagation-grid velocity, ix fastest
   const double* xpos = nullptr;       // interface node x (= velocity-grid x)
   const double* ifz[6] = {};          // interface node depths, interfaces 1..5
@@ -51,18 +53,21 @@ struct SfJob {
 // out[i] = the field's interpolated time at seafloor node i, for every job
 // (the same interpolation the entry search applies, done once per field
 // instead of once per pick).
-void tr_sf_times(const TrModel* m, const SfJob* jobs, int njobs, int nx, cudaStream_t st);
+void tr_sf_times(const TrModel& m, const SfJob* jobs, int njobs, int nx, cudaStream_t st);
 
-// Trace every pick.  Pass 1 (rows == nullptr): t_calc, valid and the number
-// of Frechet contributions of each pick (cnt).  Pass 2: the contributions
-// themselves at off[pick] (keys = pick << 32 | parameter id, 1-based).
-// entry (pass 1, may be null): per pick the receiver end of the ray (the
-// seafloor entry point of an in-water pick of phases 1-3, else the receiver)
-// and the water leg's time, 3 doubles.
-void tr_launch(const TrModel* m, const TrField* fields, const double* src_x, const double* src_z,
-               const TrPick* picks, int npick, double* t_calc, int* valid, unsigned* cnt,
-               const unsigned long long* off, unsigned long long* keys, double* vals,
-               double* entry, cudaStream_t st);
+// What a trace computes per pick: the receiver time and the valid flag;
+// these and the number of Frechet contributions (cnt); or, for the picks
+// found valid, the contributions themselves at off[pick] (keys = pick << 32 |
+// parameter id, 1-based).
+enum TrMode { kTrTimes = 0, kTrCount = 1, kTrRows = 2 };
+// m is passed to the kernel by value.  entry (not with kTrRows; may be null):
+// per pick the receiver end of the ray (the seafloor entry point of an
+// in-water pick of phases 1-3, else the receiver) and the water leg's time, 3
+// doubles.
+void tr_launch(TrMode mode, const TrModel& m, const TrField* fields, const double* src_x,
+               const double* src_z, const TrPick* picks, int npick, double* t_calc, int* valid,
+               unsigned* cnt, const unsigned long long* off, unsigned long long* keys,
+               double* vals, double* entry, cudaStream_t st);
 
 // Direct adjoint terms of the picks (the misfit's derivative with respect to
 // the node times of each pick's terminal field): for target field k
@@ -70,7 +75,7 @@ void tr_launch(const TrModel* m, const TrField* fields, const double* src_x, con
 // order, d[k][slot] += coef[p] * w for the nodes and bilinear weights through
 // which its receiver-end time is read at the entry point recorded by the
 // trace (entry, 3 doubles per pick).
-void tr_adj_picks(const TrModel* m, const TrField* fields, const TrPick* picks,
+void tr_adj_picks(const TrModel& m, const TrField* fields, const TrPick* picks,
                   const double* entry, const double* coef, const int* tgt, const int* tp,
                   const int* tpk, double* const* d, int ntgt, cudaStream_t st);
 

@@ -60,6 +60,11 @@ std::string Engine::upload_trace_tables() {
   t.dx = m.dx;
   t.tol = m.tolerance;
   t.vwater = m.vwater;
+  t.xp0 = m.xpos[0];
+  t.vdx = m.xpos[1] - m.xpos[0];
+  t.rdx = 1.0 / t.dx;
+  t.rvdx = 1.0 / t.vdx;
+  t.rvwater = 1.0 / t.vwater;
   t.vel = d_pvel_.as<double>();
   t.xpos = d_xpos_.as<double>();
   for (int k = 1; k <= 5; ++k) t.ifz[k] = ifc_buf_[k][0].as<double>();
@@ -82,7 +87,8 @@ std::string Engine::upload_trace_tables() {
     R.id = r;
     R.nnode = G.nnode;
   }
-  return put_vec(d_trmodel_, &t, 1, stream_);
+  trmodel_ = t;
+  return std::string();
 }
 
 std::string Engine::trace(const int* src, const int* phase, const double* rx, const double* rz,
@@ -136,7 +142,7 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
   if (!(e = put_vec(d_trfields_, tf.data(), tf.size(), stream_)).empty()) return e;
   if (!jobs.empty()) {
     if (!(e = put_vec(d_sfjobs_, jobs.data(), jobs.size(), stream_)).empty()) return e;
-    tr_sf_times(d_trmodel_.as<TrModel>(), d_sfjobs_.as<SfJob>(), (int)jobs.size(), m_.nx, stream_);
+    tr_sf_times(trmodel_, d_sfjobs_.as<SfJob>(), (int)jobs.size(), m_.nx, stream_);
     ++stats_.launches;
     TCK(cudaGetLastError());
   }
@@ -165,12 +171,11 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
   nnz_ = 0;
   npick_ = -1;   // no rows to hand out unless this trace completes
   if (npick > 0) {
-    const TrModel* M = d_trmodel_.as<TrModel>();
     unsigned* cnt = d_cnt_.as<unsigned>();
     TCK(cudaMemsetAsync(cnt, 0, (np + 1) * sizeof(unsigned), stream_));
-    tr_launch(M, d_trfields_.as<TrField>(), d_srcx_.as<double>(), d_srcz_.as<double>(),
-              d_picks_.as<TrPick>(), npick, d_tcalc_.as<double>(), d_valid_.as<int>(), cnt,
-              nullptr, nullptr, nullptr, d_entry_.as<double>(), stream_);
+    tr_launch(rows ? kTrCount : kTrTimes, trmodel_, d_trfields_.as<TrField>(),
+              d_srcx_.as<double>(), d_srcz_.as<double>(), d_picks_.as<TrPick>(), npick,
+              d_tcalc_.as<double>(), d_valid_.as<int>(), cnt, nullptr, nullptr, nullptr, d_entry_.as<double>(), stream_);
     ++stats_.launches;
     TCK(cudaGetLastError());
     if (!rows) {   // times only (the line search's compute_rms_after_forward)
@@ -202,8 +207,8 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
     keys2.alloc(nt * 8);
     vals2.alloc(nt * 8);
     if (!keys.p || !vals.p || !keys2.p || !vals2.p) return "device allocation failed (Frechet)";
-    tr_launch(M, d_trfields_.as<TrField>(), d_srcx_.as<double>(), d_srcz_.as<double>(),
-              d_picks_.as<TrPick>(), npick, d_tcalc_.as<double>(), d_valid_.as<int>(), cnt, off,
+    tr_launch(kTrRows, trmodel_, d_trfields_.as<TrField>(), d_srcx_.as<double>(),
+              d_srcz_.as<double>(), d_picks_.as<TrPick>(), npick, d_tcalc_.as<double>(), d_valid_.as<int>(), cnt, off,
               keys.as<unsigned long long>(), vals.as<double>(), nullptr, stream_);
     ++stats_.launches;
     TCK(cudaGetLastError());
