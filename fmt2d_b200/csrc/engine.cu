@@ -43,7 +43,12 @@ unsigned phase_fields(int mask) {
 void DevBuf::alloc(size_t n) {
   if (n <= bytes && p) return;
   free_();
-  if (cudaMalloc(&p, n < 16 ? 16 : n) != cudaSuccess) { p = nullptr; bytes = 0; return; }
+  if (cudaMalloc(&p, n < 16 ? 16 : n) != cudaSuccess) {
+    cudaGetLastError();   // the caller's to report: not the next launch check's
+    p = nullptr;
+    bytes = 0;
+    return;
+  }
   bytes = n;
 }
 
@@ -262,6 +267,7 @@ std::string Engine::forward(const double* sx, int nsrc, int phase_mask) {
       F.solved = false;
       if (!(need & (1u << tf))) continue;
       const DevRegionStore& D = reg_[kTf[tf].reg];
+      if (F.T.bytes < D.nslots * 8) rowspace_.release();
       F.T.alloc(D.nslots * 8);
       F.G.alloc(D.nslots * 16);
       F.Gout.alloc(D.nslots * 16);

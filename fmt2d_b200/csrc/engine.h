@@ -196,6 +196,15 @@ class Engine {
   DevBuf d_pvel_, d_invidx_, d_xpos_, d_picks_, d_trfields_, d_srcx_, d_srcz_,
       d_tcalc_, d_valid_, d_cnt_, d_off_, d_rowptr_, d_tmp_, d_col_, d_val_, d_sft_, d_sfjobs_,
       d_entry_;
+  // Frechet rows' workspace: sort keys and values, the pool of the rays'
+  // entries (the sort's second buffers later), its chunks' owners and counter.
+  // Kept while it is a small part of the device's memory (trace), given back
+  // when the time fields grow (forward)
+  struct RowSpace {
+    DevBuf keys, vals, ids, pvals, owner, used;
+    size_t bytes() const { return keys.bytes + vals.bytes + ids.bytes + pvals.bytes + owner.bytes; }
+    void release();
+  } rowspace_;
   int npick_ = -1, rows_ = 0;
   long long nnz_ = 0;
   double trace_ms_ = 0.0;

@@ -37,7 +37,9 @@
 // last point of a section is ever moved after it is computed), consecutive
 // segments that touch the same four parameters are merged, and the
 // contributions are written as (pick, parameter) keys.  The caller sorts
-// the keys and sums equal ones into CSR rows.
+// the keys and sums equal ones into CSR rows.  One pass traces and writes: a ray
+// takes chunks of a pool as it goes, and a gather puts them in pick order
+// (counting first cost a second trace: 57 of 130 ms on 2001 x 401 nodes).
 #include "rays.cuh"
 #include "model.h"
 #include <algorithm>
@@ -408,16 +410,17 @@ __device__ double vel_at(const TrModel& M, double px, double pz) {
          (1.0 - w1) * w2 * V(ix, iz + 1) + w1 * w2 * V(ix + 1, iz + 1);
 }
 
-// Frechet contributions of one pick, counted (kTrCount) or written (kTrRows).
+// Frechet contributions of one pick.  They are written as the ray is traced,
+// into chunks of the pool that it takes as it needs them: how many there will
+// be is not known before its end.  Without a chunk left they are only counted.
 // The pending entries are those of the last segment's cell, compacted (ids 0
 // beyond them).
 template <int MODE>
 struct Sink {
-  unsigned long long* keys;
-  double* vals;
-  unsigned long long base;   // first entry of this pick
+  TrPool pool;
+  unsigned long long chunk;  // the current chunk's first entry, ~0: none
   unsigned n;                // entries so far
-  unsigned long long row;    // pick << 32
+  int pick;
   int cell;                  // the pending entries' cell, -1: none
   int ivx, ivz;              // its column and row, from 1
   double qx, qz;             // and from 0
@@ -429,9 +432,18 @@ struct Sink {
 template <int MODE>
 __device__ __forceinline__ void sink_put(Sink<MODE>& k, int idx, double v) {
   if (idx <= 0) return;
-  if (MODE == kTrRows) {
-    k.keys[k.base + k.n] = k.row | (unsigned)idx;
-    k.vals[k.base + k.n] = v;
+  const unsigned at = k.n % kTrChunk;
+  if (at == 0) {
+    const unsigned c = atomicAdd(k.pool.used, 1u);
+    k.chunk = ~0ull;
+    if (c < k.pool.nchunks) {
+      k.pool.owner[c] = make_uint2((unsigned)k.pick, k.n / kTrChunk);
+      k.chunk = (unsigned long long)c * kTrChunk;
+    }
+  }
+  if (k.chunk != ~0ull) {
+    k.pool.ids[k.chunk + at] = idx;
+    k.pool.vals[k.chunk + at] = v;
   }
   ++k.n;
 }
@@ -472,7 +484,6 @@ __device__ __forceinline__ void segment(const TrModel& M, Sink<MODE>& k, double 
   if (shorter(d2, 1.0e-10, 1.0e-10 * 1.0e-10)) return;
   const bool same =
       inside((px - M.xp0) * M.rvdx, k.qx) && inside((pz - gzc(M, 1)) * M.rdx, k.qz);
-  if (MODE == kTrCount && same) return;   // the pending entries' parameters again
   int ivx = k.ivx, ivz = k.ivz;
   if (!same) {
     if (pz < gzc(M, 1)) return;
@@ -485,17 +496,13 @@ __device__ __forceinline__ void segment(const TrModel& M, Sink<MODE>& k, double 
     }
   }
   const int cell = (ivz - 1) * M.nx + (ivx - 1);
-  double a = 0.0, b = 0.0, c = 0.0, d = 0.0;
-  if (MODE == kTrRows) {
-    const double sl = sqrt(d2);
-    const double wx = clamp01(quot(px - M.xpos[ivx - 1], M.vdx, M.rvdx));
-    const double wz =
-        pz >= gzc(M, M.nz) ? 1.0 : clamp01(quot(pz - gzc(M, ivz), M.dx, M.rdx));
-    a = (1.0 - wx) * (1.0 - wz) * sl;
-    b = wx * (1.0 - wz) * sl;
-    c = (1.0 - wx) * wz * sl;
-    d = wx * wz * sl;
-  }
+  const double sl = sqrt(d2);
+  const double wx = clamp01(quot(px - M.xpos[ivx - 1], M.vdx, M.rvdx));
+  const double wz = pz >= gzc(M, M.nz) ? 1.0 : clamp01(quot(pz - gzc(M, ivz), M.dx, M.rdx));
+  double a = (1.0 - wx) * (1.0 - wz) * sl;
+  double b = wx * (1.0 - wz) * sl;
+  double c = (1.0 - wx) * wz * sl;
+  double d = wx * wz * sl;
   if (cell != k.cell) {
     int q0 = M.inv_idx[cell], q1 = M.inv_idx[cell + 1];
     int q2 = M.inv_idx[cell + M.nx], q3 = M.inv_idx[cell + M.nx + 1];
@@ -512,13 +519,11 @@ __device__ __forceinline__ void segment(const TrModel& M, Sink<MODE>& k, double 
     k.qx = (double)(ivx - 1);
     k.qz = (double)(ivz - 1);
   }
-  if (MODE == kTrRows) {
-    compact(k.mask, a, b, c, d);
-    k.v0 += a;
-    k.v1 += b;
-    k.v2 += c;
-    k.v3 += d;
-  }
+  compact(k.mask, a, b, c, d);
+  k.v0 += a;
+  k.v1 += b;
+  k.v2 += c;
+  k.v3 += d;
 }
 
 template <int MODE>
@@ -1011,13 +1016,12 @@ template <int MODE>
 __global__ void __launch_bounds__(kTraceThreads, 4)
     k_trace(const __grid_constant__ TrModel M, const TrField* fields, const double* src_x,
             const double* src_z, const TrPick* picks, int npick, int per, double* t_calc,
-            int* valid, unsigned* cnt, const unsigned long long* off, unsigned long long* keys,
-            double* vals, double* entry) {
+            int* valid, bool again, unsigned* cnt, TrPool pool, double* entry) {
   // (lanes without a ray go along: whole warps trace)
   const int lane = threadIdx.x & 31;
   const int p0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) +
                  lane * (int)(gridDim.x * (kTraceThreads / 32));
-  const bool mine = lane < per && p0 < npick && !(MODE == kTrRows && !valid[p0]);
+  const bool mine = lane < per && p0 < npick && !(again && !valid[p0]);
   const int p = mine ? p0 : 0;
   const TrPick pk = picks[p];
   Section sec[kMaxSec + 1];
@@ -1032,11 +1036,10 @@ __global__ void __launch_bounds__(kTraceThreads, 4)
   R.headwave = false;
   R.diffracted = false;
   Sink<MODE> sk;
-  sk.keys = keys;
-  sk.vals = vals;
-  sk.base = MODE == kTrRows ? off[p] : 0;
+  sk.pool = pool;
+  sk.chunk = ~0ull;
   sk.n = 0;
-  sk.row = (unsigned long long)p << 32;
+  sk.pick = p;
   sk.cell = -1;
   sk.ivx = sk.ivz = 1;
   sk.qx = sk.qz = -10.0;
@@ -1096,10 +1099,10 @@ __global__ void __launch_bounds__(kTraceThreads, 4)
     iface_entries(R);
     sink_flush(sk);
   }
-  if (MODE != kTrRows && mine) {
+  if (mine && !again) {
     t_calc[p] = tr;
     valid[p] = ok ? 1 : 0;
-    if (MODE == kTrCount) cnt[p] = ok ? sk.n : 0u;
+    if (MODE == kTrRows) cnt[p] = ok ? sk.n : 0u;
     if (entry) {
       entry[3 * (size_t)p] = ent_x;
       entry[3 * (size_t)p + 1] = ent_z;
@@ -1206,25 +1209,43 @@ void tr_sf_times(const TrModel& m, const SfJob* jobs, int njobs, int nx, cudaStr
   k_sf_times<<<dim3((nx + 127) / 128, njobs), 128, 0, st>>>(m, jobs, njobs, nx);
 }
 
+// One block per chunk: an entry's place is its pick's offset plus its number
+// within the pick.
+__global__ void __launch_bounds__(kTrChunk)
+    k_gather(TrPool pool, const int* valid, const unsigned* cnt, const unsigned long long* off,
+             unsigned long long* keys, double* vals) {
+  const uint2 o = pool.owner[blockIdx.x];
+  const unsigned i = o.y * kTrChunk + threadIdx.x;
+  if (!valid[o.x] || i >= cnt[o.x]) return;
+  const unsigned long long from = (unsigned long long)blockIdx.x * kTrChunk + threadIdx.x;
+  keys[off[o.x] + i] = ((unsigned long long)o.x << 32) | (unsigned)pool.ids[from];
+  vals[off[o.x] + i] = pool.vals[from];
+}
+
+void tr_gather(const TrPool& pool, unsigned nchunks, const int* valid, const unsigned* cnt,
+               const unsigned long long* off, unsigned long long* keys, double* vals,
+               cudaStream_t st) {
+  if (nchunks == 0) return;
+  k_gather<<<nchunks, kTrChunk, 0, st>>>(pool, valid, cnt, off, keys, vals);
+}
+
 void tr_launch(TrMode mode, const TrModel& m, const TrField* fields, const double* src_x,
                const double* src_z, const TrPick* picks, int npick, double* t_calc, int* valid,
-               unsigned* cnt, const unsigned long long* off, unsigned long long* keys,
-               double* vals, double* entry, cudaStream_t st) {
+               bool again, unsigned* cnt, const TrPool& pool, double* entry, cudaStream_t st) {
   // rays of a warp: as few as keep all warps resident at once
   int dev = 0, nsm = 148, blocks = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_trace<kTrRows>, kTraceThreads, 0);
   const int warps = std::max(1, nsm * std::max(1, blocks) * (kTraceThreads / 32));
-  int per = std::min(32, (npick + warps - 1) / warps);
+  const int per = std::min(32, (npick + warps - 1) / warps);
   const int need = (npick + per - 1) / per;
   const int grid = (need + kTraceThreads / 32 - 1) / (kTraceThreads / 32);
   auto run = [&](auto kernel) {
     kernel<<<grid, kTraceThreads, 0, st>>>(m, fields, src_x, src_z, picks, npick, per, t_calc,
-                                           valid, cnt, off, keys, vals, entry);
+                                           valid, again, cnt, pool, entry);
   };
   if (mode == kTrTimes) run(k_trace<kTrTimes>);
-  else if (mode == kTrCount) run(k_trace<kTrCount>);
   else run(k_trace<kTrRows>);
 }
 

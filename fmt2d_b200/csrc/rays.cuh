@@ -55,19 +55,36 @@ struct SfJob {
 // instead of once per pick).
 void tr_sf_times(const TrModel& m, const SfJob* jobs, int njobs, int nx, cudaStream_t st);
 
-// What a trace computes per pick: the receiver time and the valid flag;
-// these and the number of Frechet contributions (cnt); or, for the picks
-// found valid, the contributions themselves at off[pick] (keys = pick << 32 |
-// parameter id, 1-based).
-enum TrMode { kTrTimes = 0, kTrCount = 1, kTrRows = 2 };
-// m is passed to the kernel by value.  entry (not with kTrRows; may be null):
-// per pick the receiver end of the ray (the seafloor entry point of an
-// in-water pick of phases 1-3, else the receiver) and the water leg's time, 3
-// doubles.
+enum TrMode { kTrTimes = 0, kTrRows = 1 };
+
+// Entries of Frechet rows as the rays write them: chunk c holds entries
+// owner[c].y * kTrChunk and on of pick owner[c].x (parameter ids from 1, and
+// values).  used counts the chunks asked for, also beyond nchunks.
+constexpr unsigned kTrChunk = 128;
+struct TrPool {
+  uint2* owner = nullptr;
+  int* ids = nullptr;
+  double* vals = nullptr;
+  unsigned* used = nullptr;
+  unsigned nchunks = 0;
+};
+
+// Traces the picks: receiver time and valid flag of each, and with kTrRows
+// its entries into the pool and their number (cnt, 0 for an invalid ray).
+// again: the times and counts are there, only the entries of the valid picks
+// are wanted (the pool was too small).  m is passed to the kernel by value.
+// entry (may be null): per pick the receiver end of the ray (the seafloor entry
+// point of an in-water pick of phases 1-3, else the receiver) and the water
+// leg's time, 3 doubles.
 void tr_launch(TrMode mode, const TrModel& m, const TrField* fields, const double* src_x,
                const double* src_z, const TrPick* picks, int npick, double* t_calc, int* valid,
-               unsigned* cnt, const unsigned long long* off, unsigned long long* keys,
-               double* vals, double* entry, cudaStream_t st);
+               bool again, unsigned* cnt, const TrPool& pool, double* entry, cudaStream_t st);
+
+// Entries of the pool's first nchunks chunks to their places: pick p's entry i
+// at off[p] + i (keys = pick << 32 | parameter id).  Invalid picks' are left.
+void tr_gather(const TrPool& pool, unsigned nchunks, const int* valid, const unsigned* cnt,
+               const unsigned long long* off, unsigned long long* keys, double* vals,
+               cudaStream_t st);
 
 // Direct adjoint terms of the picks (the misfit's derivative with respect to
 // the node times of each pick's terminal field): for target field k

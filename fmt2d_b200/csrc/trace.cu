@@ -9,6 +9,7 @@
 #include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
 #include <algorithm>
+#include <cmath>
 
 namespace fmt2d {
 
@@ -20,13 +21,26 @@ namespace fmt2d {
 
 namespace {
 
-__global__ void k_keep(const unsigned long long* keys, const double* vals, int n, int* flag,
-                       int* row_cnt) {
+__global__ void k_keep(const double* vals, int n, int* flag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const bool keep = fabs(vals[i]) > 1.0e-30;
-  flag[i] = keep ? 1 : 0;
-  if (keep) atomicAdd(row_cnt + (int)(keys[i] >> 32), 1);
+  if (i > n) return;
+  flag[i] = i < n && fabs(vals[i]) > 1.0e-30 ? 1 : 0;
+}
+
+// Row starts: the kept entries before a pick's first key (counting them per
+// pick with atomics took 2.8 ms for 22 million entries of 30276 picks).
+__global__ void k_row_starts(const unsigned long long* keys, const int* pos, int n, int npick,
+                             int* row_ptr) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p > npick) return;
+  const unsigned long long key = (unsigned long long)p << 32;
+  int a = 0, b = n;
+  while (a < b) {
+    const int m = a + (b - a) / 2;
+    if (keys[m] < key) a = m + 1;
+    else b = m;
+  }
+  row_ptr[p] = pos[a];
 }
 
 __global__ void k_scatter_rows(const unsigned long long* keys, const double* vals,
@@ -89,6 +103,10 @@ std::string Engine::upload_trace_tables() {
   }
   trmodel_ = t;
   return std::string();
+}
+
+void Engine::RowSpace::release() {
+  for (DevBuf* b : {&keys, &vals, &ids, &pvals, &owner, &used}) b->free_();
 }
 
 std::string Engine::trace(const int* src, const int* phase, const double* rx, const double* rz,
@@ -173,10 +191,51 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
   if (npick > 0) {
     unsigned* cnt = d_cnt_.as<unsigned>();
     TCK(cudaMemsetAsync(cnt, 0, (np + 1) * sizeof(unsigned), stream_));
-    tr_launch(rows ? kTrCount : kTrTimes, trmodel_, d_trfields_.as<TrField>(),
-              d_srcx_.as<double>(), d_srcz_.as<double>(), d_picks_.as<TrPick>(), npick,
-              d_tcalc_.as<double>(), d_valid_.as<int>(), cnt, nullptr, nullptr, nullptr, d_entry_.as<double>(), stream_);
-    ++stats_.launches;
+    // the pool: entries of a ray as long as its offset and the model's depth
+    // twice (four a cell); where that is too little, or memory is short, the
+    // rays that count their entries are traced again into one of the right size
+    RowSpace& W = rowspace_;
+    size_t chunks = 0;
+    TrPool pool;
+    auto set_pool = [&](size_t n) {
+      W.ids.alloc(n * kTrChunk * sizeof(unsigned long long));   // (sort keys later)
+      W.pvals.alloc(n * kTrChunk * sizeof(double));
+      W.owner.alloc(n * sizeof(uint2));
+      const bool ok = W.ids.p && W.pvals.p && W.owner.p;
+      pool.ids = W.ids.as<int>();
+      pool.vals = W.pvals.as<double>();
+      pool.owner = W.owner.as<uint2>();
+      pool.nchunks = ok ? (unsigned)std::min({W.ids.bytes / (kTrChunk * 8),
+                                              W.pvals.bytes / (kTrChunk * 8),
+                                              W.owner.bytes / sizeof(uint2),
+                                              (size_t)0x7fffffff}) : 0u;
+      return ok;
+    };
+    if (rows) {
+      double len = 0.0;
+      for (int i = 0; i < npick; ++i)
+        len += std::min(std::fabs(rx[i] - src_x_[src[i]]) / m_.dx, (double)m_.nx) + 2.0 * m_.nz;
+      if (!(len >= 0.0)) len = 0.0;   // (a receiver that is not a number)
+      chunks = (size_t)(4.0 * len / kTrChunk) + (size_t)npick;
+      W.used.alloc(sizeof(unsigned));
+      if (!W.used.p) return "device allocation failed (Frechet)";
+      size_t free_b = 0, total_b = 0;
+      TCK(cudaMemGetInfo(&free_b, &total_b));
+      const size_t fit = (free_b / 4 + W.ids.bytes + W.pvals.bytes + W.owner.bytes) /
+                         (kTrChunk * 16 + sizeof(uint2));
+      // (no memory for a pool: the rays are counted)
+      set_pool(std::min({chunks, fit, (size_t)(0x7fffffffu / kTrChunk) + npick}));
+      pool.used = W.used.as<unsigned>();
+      TCK(cudaMemsetAsync(W.used.p, 0, sizeof(unsigned), stream_));
+    }
+    auto launch = [&](bool again) {
+      tr_launch(rows ? kTrRows : kTrTimes, trmodel_, d_trfields_.as<TrField>(),
+                d_srcx_.as<double>(), d_srcz_.as<double>(), d_picks_.as<TrPick>(), npick,
+                d_tcalc_.as<double>(), d_valid_.as<int>(), again, cnt, pool,
+                d_entry_.as<double>(), stream_);
+      ++stats_.launches;
+    };
+    launch(false);
     TCK(cudaGetLastError());
     if (!rows) {   // times only (the line search's compute_rms_after_forward)
       TCK(cudaMemcpyAsync(t_calc, d_tcalc_.p, (size_t)npick * 8, cudaMemcpyDeviceToHost, stream_));
@@ -190,26 +249,50 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
       if (nnz) *nnz = 0;
       return std::string();
     }
+    auto temp = [&](size_t bytes) {
+      d_tmp_.alloc(std::max<size_t>(bytes, 16));
+      return d_tmp_.p != nullptr;
+    };
     // offsets of each pick's contributions (64-bit: long rays times many picks)
     unsigned long long* off = d_off_.as<unsigned long long>();
     size_t tmp_bytes = 0;
     TCK(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt, off, npick + 1, stream_));
-    d_tmp_.alloc(std::max<size_t>(tmp_bytes, 16));
+    if (!temp(tmp_bytes)) return "device allocation failed (Frechet)";
     TCK(cub::DeviceScan::ExclusiveSum(d_tmp_.p, tmp_bytes, cnt, off, npick + 1, stream_));
     unsigned long long total = 0;
+    unsigned used = 0;
     TCK(cudaMemcpyAsync(&total, off + npick, sizeof(total), cudaMemcpyDeviceToHost, stream_));
+    TCK(cudaMemcpyAsync(&used, W.used.p, sizeof(used), cudaMemcpyDeviceToHost, stream_));
     TCK(cudaStreamSynchronize(stream_));
     if (total >= 0x7fffffffull) return "too many Frechet contributions for 32-bit CSR";
-    const size_t nt = std::max<size_t>((size_t)total, 1);
-    DevBuf keys, vals, keys2, vals2;
-    keys.alloc(nt * 8);
-    vals.alloc(nt * 8);
-    keys2.alloc(nt * 8);
-    vals2.alloc(nt * 8);
-    if (!keys.p || !vals.p || !keys2.p || !vals2.p) return "device allocation failed (Frechet)";
-    tr_launch(kTrRows, trmodel_, d_trfields_.as<TrField>(), d_srcx_.as<double>(),
-              d_srcz_.as<double>(), d_picks_.as<TrPick>(), npick, d_tcalc_.as<double>(), d_valid_.as<int>(), cnt, off,
-              keys.as<unsigned long long>(), vals.as<double>(), nullptr, stream_);
+    struct Keep {   // the workspace stays only while it is small, whatever the way out
+      RowSpace& w;
+      ~Keep() {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || w.bytes() > total_b / 16)
+          w.release();
+      }
+    } keep{W};
+    if (used > pool.nchunks) {
+      if (!set_pool((size_t)total / kTrChunk + npick)) return "device allocation failed (Frechet)";
+      TCK(cudaMemsetAsync(W.used.p, 0, sizeof(unsigned), stream_));
+      launch(true);
+      TCK(cudaGetLastError());
+      TCK(cudaMemcpyAsync(&used, W.used.p, sizeof(used), cudaMemcpyDeviceToHost, stream_));
+      TCK(cudaStreamSynchronize(stream_));
+      if (used > pool.nchunks) return "ray entries out of step with their count";
+    }
+    const size_t nt = std::max<size_t>((size_t)total, 2);
+    W.keys.alloc(nt * 8);
+    W.vals.alloc(nt * 8);
+    W.ids.alloc(nt * 8);
+    W.pvals.alloc(nt * 8);
+    if (!W.keys.p || !W.vals.p || !W.ids.p || !W.pvals.p)
+      return "device allocation failed (Frechet)";
+    cub::DoubleBuffer<unsigned long long> kb(W.keys.as<unsigned long long>(),
+                                             W.ids.as<unsigned long long>());
+    cub::DoubleBuffer<double> vb(W.vals.as<double>(), W.pvals.as<double>());
+    tr_gather(pool, used, d_valid_.as<int>(), cnt, off, kb.Current(), vb.Current(), stream_);
     ++stats_.launches;
     TCK(cudaGetLastError());
     const int n = (int)total;
@@ -218,61 +301,41 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
     // stable sort by (pick, parameter): contributions of one entry stay in
     // segment order
     size_t sb = 0;
-    TCK(cub::DeviceRadixSort::SortPairs(nullptr, sb, keys.as<unsigned long long>(),
-                                        keys2.as<unsigned long long>(), vals.as<double>(),
-                                        vals2.as<double>(), n, 0, end_bit, stream_));
-    d_tmp_.alloc(std::max<size_t>(sb, 16));
-    TCK(cub::DeviceRadixSort::SortPairs(d_tmp_.p, sb, keys.as<unsigned long long>(),
-                                        keys2.as<unsigned long long>(), vals.as<double>(),
-                                        vals2.as<double>(), n, 0, end_bit, stream_));
+    TCK(cub::DeviceRadixSort::SortPairs(nullptr, sb, kb, vb, n, 0, end_bit, stream_));
+    if (!temp(sb)) return "device allocation failed (Frechet sort)";
+    TCK(cub::DeviceRadixSort::SortPairs(d_tmp_.p, sb, kb, vb, n, 0, end_bit, stream_));
     // sum equal keys
-    DevBuf nruns;
-    nruns.alloc(16);
+    unsigned long long* keys = kb.Alternate();
+    double* vals = vb.Alternate();
+    int* nruns = W.used.as<int>();
     size_t rb = 0;
-    TCK(cub::DeviceReduce::ReduceByKey(nullptr, rb, keys2.as<unsigned long long>(),
-                                       keys.as<unsigned long long>(), vals2.as<double>(),
-                                       vals.as<double>(), nruns.as<int>(), ::cuda::std::plus<>{}, n, stream_));
-    d_tmp_.alloc(std::max<size_t>(rb, 16));
-    TCK(cub::DeviceReduce::ReduceByKey(d_tmp_.p, rb, keys2.as<unsigned long long>(),
-                                       keys.as<unsigned long long>(), vals2.as<double>(),
-                                       vals.as<double>(), nruns.as<int>(), ::cuda::std::plus<>{}, n, stream_));
+    TCK(cub::DeviceReduce::ReduceByKey(nullptr, rb, kb.Current(), keys, vb.Current(), vals, nruns,
+                                       ::cuda::std::plus<>{}, n, stream_));
+    if (!temp(rb)) return "device allocation failed (Frechet sums)";
+    TCK(cub::DeviceReduce::ReduceByKey(d_tmp_.p, rb, kb.Current(), keys, vb.Current(), vals, nruns,
+                                       ::cuda::std::plus<>{}, n, stream_));
     int nu = 0;
-    TCK(cudaMemcpyAsync(&nu, nruns.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    TCK(cudaMemcpyAsync(&nu, nruns, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     TCK(cudaStreamSynchronize(stream_));
-    // drop zero entries, count each row, place the survivors
-    DevBuf flag, pos, rcnt;
-    flag.alloc((size_t)std::max(nu, 1) * 4);
-    pos.alloc((size_t)std::max(nu, 1) * 4);
-    rcnt.alloc((np + 1) * 4);
-    if (!flag.p || !pos.p || !rcnt.p) return "device allocation failed (Frechet rows)";
-    TCK(cudaMemsetAsync(rcnt.p, 0, (np + 1) * 4, stream_));
-    if (nu > 0)
-      k_keep<<<(nu + 255) / 256, 256, 0, stream_>>>(keys.as<unsigned long long>(),
-                                                     vals.as<double>(), nu, flag.as<int>(),
-                                                     rcnt.as<int>());
+    // drop zero entries, find each row's start, place the survivors
+    int *flag = (int*)kb.Current(), *pos = (int*)vb.Current();   // (nu + 1 <= 2 nt)
+    k_keep<<<nu / 256 + 1, 256, 0, stream_>>>(vals, nu, flag);
     ++stats_.launches;
     size_t qb = 0;
-    TCK(cub::DeviceScan::ExclusiveSum(nullptr, qb, flag.as<int>(), pos.as<int>(), std::max(nu, 1),
-                                      stream_));
-    size_t qb2 = 0;
-    TCK(cub::DeviceScan::ExclusiveSum(nullptr, qb2, rcnt.as<int>(), d_rowptr_.as<int>(),
-                                      npick + 1, stream_));
-    d_tmp_.alloc(std::max<size_t>(std::max(qb, qb2), 16));
-    if (nu > 0)
-      TCK(cub::DeviceScan::ExclusiveSum(d_tmp_.p, qb, flag.as<int>(), pos.as<int>(), nu, stream_));
-    TCK(cub::DeviceScan::ExclusiveSum(d_tmp_.p, qb2, rcnt.as<int>(), d_rowptr_.as<int>(),
-                                      npick + 1, stream_));
+    TCK(cub::DeviceScan::ExclusiveSum(nullptr, qb, flag, pos, nu + 1, stream_));
+    if (!temp(qb)) return "device allocation failed (Frechet rows)";
+    TCK(cub::DeviceScan::ExclusiveSum(d_tmp_.p, qb, flag, pos, nu + 1, stream_));
+    k_row_starts<<<npick / 256 + 1, 256, 0, stream_>>>(keys, pos, nu, npick, d_rowptr_.as<int>());
+    ++stats_.launches;
     int kept = 0;
-    TCK(cudaMemcpyAsync(&kept, d_rowptr_.as<int>() + npick, sizeof(int), cudaMemcpyDeviceToHost,
-                        stream_));
+    TCK(cudaMemcpyAsync(&kept, pos + nu, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     TCK(cudaStreamSynchronize(stream_));
     d_col_.alloc((size_t)std::max(kept, 1) * 4);
     d_val_.alloc((size_t)std::max(kept, 1) * 8);
     if (!d_col_.p || !d_val_.p) return "device allocation failed (Frechet rows)";
     if (nu > 0)
-      k_scatter_rows<<<(nu + 255) / 256, 256, 0, stream_>>>(
-          keys.as<unsigned long long>(), vals.as<double>(), flag.as<int>(), pos.as<int>(), nu,
-          d_col_.as<int>(), d_val_.as<double>());
+      k_scatter_rows<<<(nu + 255) / 256, 256, 0, stream_>>>(keys, vals, flag, pos, nu,
+                                                            d_col_.as<int>(), d_val_.as<double>());
     ++stats_.launches;
     TCK(cudaGetLastError());
     nnz_ = kept;
