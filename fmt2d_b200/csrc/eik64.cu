@@ -26,6 +26,7 @@
 // Arithmetic is FP64 with the reference's expression order; this file is
 // compiled with --fmad=false so candidate times are bit-identical to the
 // FP64 restatement's.
+#include <math_constants.h>
 #include <algorithm>
 #include <climits>
 #include <mutex>
@@ -734,14 +735,32 @@ __device__ __forceinline__ void list_start(const Fld64& F, unsigned s) {
 }
 
 // Fixed-point check of every node (window ignored): a node whose update
-// would change it is listed and counted.
+// would change it is listed and counted.  Nodes at an interface are evaluated
+// by evaluate(), on the state as it was unpacked; the regular ones, which are
+// nearly all and cost a dozen roots and quotients there, by reg_best on the
+// records the state came from (60 fields of 800,000 nodes:).
 __global__ void k_verify(Fld64* fields, int nf) {
   const Fld64& F = fields[blockIdx.y];
   const int ns = F.nslots();
+  const double rdx = 1.0 / F.dx;
+  constexpr uint32_t kPlain = kInRegion | kUpdatable | kFullyRegular;
   unsigned nbad = 0;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
-    if ((s % F.pitch) >= F.nx) continue;
-    const NewV nv = evaluate(F, s);
+    const int row = s / F.pitch, col = s - row * F.pitch;
+    if (col >= F.nx) continue;
+    NewV nv;
+    if ((F.code[s] & kPlain) == kPlain && row < F.H) {
+      if (s == F.frozen_slot) continue;
+      const Rec me = load_rec(F, s);
+      Self self;
+      self.T = me.T;
+      self.g = make_double2(me.gx, me.gz);
+      self.fl = F.fl[s];
+      const RegBest rb = reg_best<false>(F, rdx, s, row, col, fabs(me.v), 15u);
+      nv = settle(F, s, rb.t, rb.gx, rb.gz, false, rb.key != kNoKey && !(rb.key & 1), rb.t, self);
+    } else {
+      nv = evaluate(F, s);
+    }
     if (nv.write) {
       ++nbad;
       list_start(F, (unsigned)s);
@@ -919,8 +938,20 @@ __global__ void k_seed_iface(Fld64* fields, const Seed64* descs, int nd, int nx)
 __global__ void k_clock(Fld64* fields, int nf, const double* step) {
   Fld64& F = fields[blockIdx.x];
   const int ns = (F.H + 2) * F.pitch;
+  // the flags, sixteen slots a load (one block reads a field: a slot a load
+  // took 1.2 ms for 60 fields of 800,000)
   double mn = kHugeD;
-  for (int s = threadIdx.x; s < ns; s += blockDim.x)
+  const int nv = ns / 16;
+  const uint4* fl = reinterpret_cast<const uint4*>(F.fl);
+  constexpr unsigned kAny = kFlSeed * 0x01010101u;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+    const uint4 w = fl[i];
+    if (!((w.x | w.y | w.z | w.w) & kAny)) continue;
+    for (int s = 16 * i; s < 16 * i + 16; ++s)
+      if (F.fl[s] & kFlSeed) mn = fmin(mn, F.T[s]);
+  }
+  for (int s = 16 * nv + threadIdx.x; s < ns; s += blockDim.x)
     if (F.fl[s] & kFlSeed) mn = fmin(mn, F.T[s]);
   __shared__ double sm[32];
 #pragma unroll
@@ -969,30 +1000,64 @@ __global__ void k_water_fix(Fld64* fields, const int* upward, int nf) {
   if (bad) F.Gout[st] = F.Gout[sb];
 }
 
-// PmP head-wave min-plus sweep along the Moho (inversion2d.f90:4294-4409), one
-// field per thread; node table and velocities are precomputed per model.
+// PmP head-wave min-plus sweep along the Moho (inversion2d.f90:4294-4409), a
+// block per field; node table and velocities are precomputed per model.  The
+// two sweeps are chains over the nodes (their sums round in that order): one
+// thread runs them from shared memory, a batch of nodes at a time, and all
+// else is spread over the block (one thread per field took 7.5 ms for 2001
+// nodes, the fields' loads one after the other).
 // The solved times the sweep replaces are saved first (pre, nx per field:
 // the adjoint re-derives each node's winning update from them).
-__global__ void k_headwave(Fld64* fields, const int* hw_slot, const double* hw_v, double dx_if,
-                           int nx, double* scratch, const int* which, int nsel,
-                           double* const* pre) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsel) return;
+constexpr int kHwBatch = 1024;
+__global__ void __launch_bounds__(256)
+    k_headwave(Fld64* fields, const int* hw_slot, const double* hw_v, double dx_if, int nx,
+               double* scratch, const int* which, double* const* pre) {
+  const int q = blockIdx.x, tid = threadIdx.x;
   Fld64& F = fields[which[q]];
   double* th = scratch + (size_t)q * nx;
-  for (int n = 0; n < nx; ++n) th[n] = hw_slot[n] >= 0 ? F.T[hw_slot[n]] : kHugeD;
-  if (pre && pre[q])
-    for (int n = 0; n < nx; ++n) pre[q][n] = th[n];
-  for (int n = 1; n < nx; ++n)
-    if (hw_v[n] > 0.0) th[n] = fmin(th[n], th[n - 1] + dx_if / hw_v[n]);
-  for (int n = nx - 2; n >= 0; --n)
-    if (hw_v[n] > 0.0) th[n] = fmin(th[n], th[n + 1] + dx_if / hw_v[n]);
-  for (int n = 0; n < nx; ++n) {
+  double* keep = pre ? pre[q] : nullptr;
+  __shared__ double s_t[kHwBatch], s_d[kHwBatch];
+  __shared__ double s_last;
+  // dir 1: left to right, the nodes' times from the field; -1: back, from th
+  auto sweep = [&](int dir) {
+    for (int b = 0; b < nx; b += kHwBatch) {
+      const int m = min(kHwBatch, nx - b);
+      for (int i = tid; i < m; i += blockDim.x) {
+        const int n = dir > 0 ? b + i : nx - 1 - (b + i);
+        double t;
+        if (dir > 0) {
+          t = hw_slot[n] >= 0 ? F.T[hw_slot[n]] : kHugeD;
+          if (keep) keep[n] = t;
+        } else {
+          t = th[n];
+        }
+        s_t[i] = t;
+        // (a node without a velocity keeps its time)
+        s_d[i] = hw_v[n] > 0.0 ? dx_if / hw_v[n] : CUDART_INF;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        double t = b ? s_last : s_t[0];
+#pragma unroll 8
+        for (int i = b ? 0 : 1; i < m; ++i) {
+          t = fmin(s_t[i], t + s_d[i]);
+          s_t[i] = t;
+        }
+        s_last = t;
+      }
+      __syncthreads();
+      for (int i = tid; i < m; i += blockDim.x) th[dir > 0 ? b + i : nx - 1 - (b + i)] = s_t[i];
+      __syncthreads();
+    }
+  };
+  sweep(1);
+  sweep(-1);
+  for (int n = tid; n < nx; n += blockDim.x) {
     const int s = hw_slot[n];
-    if (s < 0) continue;
-    if (th[n] < F.T[s] - 1.0e-10) F.T[s] = th[n];
+    if (s >= 0 && th[n] < F.T[s] - 1.0e-10) F.T[s] = th[n];
   }
-  for (int n = 0; n < nx; ++n) {
+  __syncthreads();
+  for (int n = tid; n < nx; n += blockDim.x) {
     const int s = hw_slot[n];
     if (s < 0 || F.T[s] >= kReachD) continue;
     if (!(F.code[s] & kIfaceNode)) {
@@ -1043,7 +1108,7 @@ void e64_seed_iface(Fld64* f, const Seed64* d, int nd, int nx, cudaStream_t st) 
 void e64_start(Fld64* f, int nf, size_t max_slots, const double* step, cudaStream_t st) {
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 256);
   k_queue_seeds<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
-  k_clock<<<nf, 256, 0, st>>>(f, nf, step);
+  k_clock<<<nf, 1024, 0, st>>>(f, nf, step);
 }
 int e64_tiles(const Fld64& f) { return tiles_of(f); }
 int e64_tiles_max() { return kTilesMax; }
@@ -1139,7 +1204,7 @@ void e64_finish(Fld64* f, int nf, size_t max_slots, const int* water_up, cudaStr
 void e64_headwave(Fld64* f, const int* hw_slot, const double* hw_v, double dx_if, int nx,
                   double* scratch, const int* which, int nsel, double* const* pre,
                   cudaStream_t st) {
-  k_headwave<<<(nsel + 31) / 32, 32, 0, st>>>(f, hw_slot, hw_v, dx_if, nx, scratch, which, nsel, pre);
+  k_headwave<<<nsel, 256, 0, st>>>(f, hw_slot, hw_v, dx_if, nx, scratch, which, pre);
 }
 void e64_export(const double* T, const double2* G, const int* slot_of_node, int nnode, double* oT,
                 double* ogx, double* ogz, cudaStream_t st) {
