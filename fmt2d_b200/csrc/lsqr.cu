@@ -108,7 +108,49 @@ __device__ __forceinline__ double lap_at(const LsqrDev& d, const double* x, int 
   return ((0.0 + x[j - 1]) + x[j + 1]) - 2.0 * x[j];
 }
 
-// sum_k val[k] * x[idx[k]] over [k0, k1), lanes strided, warp-reduced.
+// What bounds the products with A and its transpose: reading the entries once
+// each (12 bytes; x stays in L2), so what counts is entries in flight: a lane
+// asks for eight before it uses the first.
+constexpr int kBatch = 8, kSpan = 32 * kBatch;   // a lane's entries, a warp's
+
+// A warp's next entries: entry k + 32*i and the x it multiplies, for its lane.
+// Entries that are not there come with v = 0 and x = 0.
+__device__ __forceinline__ void entries(const int* __restrict__ idx,
+                                        const double* __restrict__ val, int k, int k1,
+                                        const double* __restrict__ x, int lim, double* v,
+                                        double* xs) {
+  int j[kBatch];
+#pragma unroll
+  for (int i = 0; i < kBatch; ++i) {
+    const bool in = k + 32 * i < k1;
+    j[i] = in ? __ldg(idx + k + 32 * i) : lim;
+    v[i] = in ? __ldg(val + k + 32 * i) : 0.0;
+  }
+#pragma unroll
+  for (int i = 0; i < kBatch; ++i) {
+    xs[i] = j[i] < lim ? x[j[i]] : 0.0;
+    if (!(j[i] < lim)) v[i] = 0.0;
+  }
+}
+
+// sum_k val[k] * x[idx[k]] over [k0, k1): a long row, the whole warp on it;
+// per lane its even and its odd entries, then the lanes.
+__device__ __forceinline__ double long_dot(const int* __restrict__ idx,
+                                           const double* __restrict__ val, int k0, int k1,
+                                           const double* __restrict__ x, int lim) {
+  double a0 = 0.0, a1 = 0.0, v[kBatch], xs[kBatch];
+  for (int k = k0; k < k1; k += kSpan) {
+    entries(idx, val, k + (int)(threadIdx.x & 31), k1, x, lim, v, xs);
+#pragma unroll
+    for (int i = 0; i < kBatch; i += 2) {
+      a0 += v[i] * xs[i];
+      a1 += v[i + 1] * xs[i + 1];
+    }
+  }
+  return warp_sum(a0 + a1);
+}
+
+// The same with two entries in flight, for the layout of smooth_type 3 (rows_log).
 __device__ __forceinline__ double warp_dot(const int* __restrict__ idx,
                                            const double* __restrict__ val, int k0, int k1,
                                            const double* __restrict__ x, int lim) {
@@ -126,6 +168,65 @@ __device__ __forceinline__ double warp_dot(const int* __restrict__ idx,
     if (j0 < lim) a0 += __ldg(val + k) * x[j0];
   }
   return warp_sum(a0 + a1);
+}
+// Short rows (a parameter's column, a smoothing row): a warp takes 2^lc
+// consecutive rows j0.. (below jn), whose entries lie side by side, so that it
+// reads them as one long row whatever their lengths; the products go through
+// shared memory (kSpan doubles a warp) and each row is summed by the 32 >> lc
+// lanes that own it, which get its sum.  A warp per row left most lanes idle
+// (21 entries a column) and the epilogue to one lane: 742,000 columns, 15
+// million entries: 0.41 -> 0.10 ms, the epilogue a lane a row too.  The rows of A
+// themselves, 640 entries each, are long_dot's: 0.125 -> 0.07 ms.
+__device__ __forceinline__ double rows_dot(const int* __restrict__ rp,
+                                           const int* __restrict__ idx,
+                                           const double* __restrict__ val, int j0, int jn, int lc,
+                                           const double* __restrict__ x, int lim, double* sm) {
+  if (lc < 0) return warp_dot(idx, val, rp[j0], rp[j0 + 1], x, lim);
+  if (lc == 0) return long_dot(idx, val, rp[j0], rp[j0 + 1], x, lim);
+  const int lane = threadIdx.x & 31, per = 32 >> lc;
+  const int c = lane / per, sub = lane & (per - 1);
+  const int je = min(j0 + (1 << lc), jn);
+  const int a = rp[min(j0 + c, je)], b = rp[min(j0 + c + 1, je)];
+  const int k0 = __shfl_sync(0xffffffffu, a, 0), k1 = __shfl_sync(0xffffffffu, b, 31);
+  double acc = 0.0, p[kBatch], xs[kBatch];
+  for (int k = k0; k < k1; k += kSpan) {
+    const int ke = min(k + kSpan, k1);
+    entries(idx, val, k + lane, ke, x, lim, p, xs);
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) p[i] *= xs[i];
+    // a row that has all of these: the warp sums them
+    const unsigned one = __ballot_sync(0xffffffffu, sub == 0 && a <= k && b >= ke);
+    if (one) {
+      const double s = warp_sum(((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])));
+      if (lane == __ffs(one) - 1) acc += s;
+      continue;
+    }
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) sm[32 * i + lane] = p[i];
+    __syncwarp();
+    const int e = min(b, ke);
+    for (int q = max(a, k) + sub; q < e; q += per) acc += sm[q - k];
+    __syncwarp();
+  }
+  for (int o = per >> 1; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
+// log2 of the rows a warp takes: as many as keep every warp busy.  The layout
+// of smooth_type 3, the inversion's usual one, keeps a warp a row and the order
+// of every sum (-1): the line search's rays are traced in its solution, and a
+// ray can turn on the last bit.
+template <int ST>
+__device__ __forceinline__ int rows_log(const LsqrDev& d, int nwarp) {
+  if (ST == 3) return -1;
+  int lc = 0;
+  while (lc < 5 && (d.np >> (lc + 1)) >= nwarp) ++lc;
+  return lc;
+}
+
+__device__ __forceinline__ double* warp_span() {
+  __shared__ double sm[kLsThreads / 32][kSpan];
+  return sm[threadIdx.x >> 5];
 }
 
 // The right-hand side's norm (every block passes its partial sum of squares):
@@ -261,9 +362,11 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_adj(LsqrDev d) {
   const double* uL = d.u + d.nd;
   const double* uD = d.u + d.nd + d.np;
   double ss = 0.0;
-  for (int j = warp; j < d.np; j += nwarp) {
-    const double g = warp_dot(d.crow, d.cval, d.cp[j], d.cp[j + 1], d.u, d.nd);
-    if (lane == 0) {
+  const int lc = rows_log<1>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
+  for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
+    const double g = rows_dot(d.cp, d.crow, d.cval, j0, d.np, lc, d.u, d.nd, warp_span());
+    const int j = j0 + lane / per;
+    if ((lane & (per - 1)) == 0 && j < d.np) {
       double atu = g / bsc;
       atu = atu + (w_smooth(d, j) * lap_at(d, uL, j)) / bsc;
       atu = atu + (w_damp(d, j) * uD[j]) / bsc;
@@ -291,7 +394,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_fwd(LsqrDev d) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarp = (gridDim.x * blockDim.x) >> 5;
     for (int i = warp; i < d.nd; i += nwarp) {
-      const double g = warp_dot(d.col, d.val, d.rp[i], d.rp[i + 1], d.v, d.np);
+      const double g = long_dot(d.col, d.val, d.rp[i], d.rp[i + 1], d.v, d.np);
       if (lane == 0) {
         const double un = g / asc - alpha * (d.u[i] / bsc);
         d.u[i] = un;
@@ -323,43 +426,45 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_fwd(LsqrDev d) {
 // rows) | damping]; adjoint L and R_i.  Masked velocity rows are zero in
 // every block (inversion2d.f90:6608-6736, 6753-6851, 6883-7120).
 
-// Row j of A times x, warp-cooperative (every lane gets the sum).
-__device__ __forceinline__ double row_dot(const SpRows& A, int j, const double* x, int np) {
-  if (!A.rp) return 0.0;
-  return warp_dot(A.col, A.val, A.rp[j], A.rp[j + 1], x, np);
+// Rows j0.. of A times x (rows_dot; 0 without a matrix).
+__device__ __forceinline__ double row_dots(const LsqrDev& d, const SpRows& A, int j0, int lc,
+                                           const double* x) {
+  return A.rp ? rows_dot(A.rp, A.col, A.val, j0, d.np, lc, x, d.np, warp_span()) : 0.0;
 }
 
 __device__ __forceinline__ double* damp_block(const LsqrDev& d) {
   return d.u + d.nd + (d.stype == 2 ? 2 : 1) * (size_t)d.np;
 }
 
-// Rows j of the smoothing blocks applied to x (unweighted by a scale):
-// s1 (the first block), s2 (the R_v block of smooth_type 2).  Warp-uniform j.
-__device__ __forceinline__ void smooth_rows(const LsqrDev& d, const double* x, int j, double* s1,
-                                            double* s2) {
-  *s2 = 0.0;
-  if (d.stype == 3) {
-    if (j < d.nvp) {
-      *s1 = w_smooth(d, j) * lap_at(d, x, j);
-    } else {
-      const double h = row_dot(d.ri, j, x, d.np);
-      *s1 = d.ws_i > 0.0 ? d.ws_i * h : 0.0;
-    }
+// Rows j0.. of the smoothing blocks applied to x (unweighted by a scale), of
+// the lane's row j: s1 (the first block), s2 (the R_v block of smooth_type 2).
+template <int ST>
+__device__ __forceinline__ void smooth_rows(const LsqrDev& d, const double* x, int j0, int lc,
+                                            int j, double* s1, double* s2) {
+  *s1 = *s2 = 0.0;
+  const bool iface = j0 + (lc < 0 ? 1 : 1 << lc) > d.nvp;   // some of the rows (the same in a warp)
+  if (ST == 3) {
+    const double h = iface ? row_dots(d, d.ri, j0, lc, x) : 0.0;
+    if (j >= d.np) return;
+    if (j < d.nvp) *s1 = w_smooth(d, j) * lap_at(d, x, j);
+    else *s1 = d.ws_i > 0.0 ? d.ws_i * h : 0.0;
     return;
   }
-  const double h = row_dot(d.rh, j, x, d.np), v = row_dot(d.rv, j, x, d.np);
+  const double h = row_dots(d, d.rh, j0, lc, x), v = row_dots(d, d.rv, j0, lc, x);
+  const bool ri = d.ws_i > 0.0 && d.ri.rp;
+  const double hi = ri && iface ? row_dots(d, d.ri, j0, lc, x) : 0.0;
+  if (j >= d.np) return;
   if (j < d.nvp) {
     const bool m = d.mask[j];
     *s1 = d.ws_v * (m ? 0.0 : h);
     *s2 = d.ws_v * (m ? 0.0 : v);
   } else {
-    const bool ri = d.ws_i > 0.0 && d.ri.rp;
-    const double hi = ri ? row_dot(d.ri, j, x, d.np) : 0.0;
     *s1 = ri ? d.ws_i * hi : 0.0;
     *s2 = d.ws_v * v;
   }
 }
 
+template <int ST>
 __global__ void __launch_bounds__(kLsThreads) k_ls_init_u_g(LsqrDev d) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31, warp = tid >> 5, nwarp = nth >> 5;
@@ -371,13 +476,15 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_init_u_g(LsqrDev d) {
   }
   double* u1 = d.u + d.nd;
   double* u2 = u1 + d.np;
-  for (int j = warp; j < d.np; j += nwarp) {
+  const int lc = rows_log<ST>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
+  for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
+    const int j = j0 + lane / per;
     double s1, s2;
-    smooth_rows(d, d.dm_sum, j, &s1, &s2);
-    if (lane == 0) {
+    smooth_rows<ST>(d, d.dm_sum, j0, lc, j, &s1, &s2);
+    if ((lane & (per - 1)) == 0 && j < d.np) {
       u1[j] = -s1;
       ss += s1 * s1;
-      if (d.stype == 2) {
+      if (ST == 2) {
         u2[j] = -s2;
         ss += s2 * s2;
       }
@@ -392,6 +499,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_init_u_g(LsqrDev d) {
   init_u_tail(d, ss);
 }
 
+template <int ST>
 __global__ void __launch_bounds__(kLsThreads) k_ls_adj_g(LsqrDev d) {
   const int state = d.sc->state;
   if (state != kLsInit && state != kLsRun) return;
@@ -405,31 +513,38 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_adj_g(LsqrDev d) {
   const double* u2 = u1 + d.np;
   const double* uD = damp_block(d);
   double ss = 0.0;
-  for (int j = warp; j < d.np; j += nwarp) {
-    const double g = warp_dot(d.crow, d.cval, d.cp[j], d.cp[j + 1], d.u, d.nd);
-    double a1, a2 = 0.0, ai = 0.0;
+  const int lc = rows_log<ST>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
+  for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
+    const int j = j0 + lane / per;
+    const bool mine = (lane & (per - 1)) == 0 && j < d.np;
+    const bool iface = j0 + (lc < 0 ? 1 : 1 << lc) > d.nvp;   // some of the rows (the same in a warp)
+    const double g = rows_dot(d.cp, d.crow, d.cval, j0, d.np, lc, d.u, d.nd, warp_span());
+    double a1 = 0.0, a2 = 0.0, ai = 0.0;
     bool has_i = false;
-    if (d.stype == 3) {
-      if (j < d.nvp) {
-        a1 = w_smooth(d, j) * lap_at(d, u1, j);
-      } else {
-        const double h = row_dot(d.ri, j, u1, d.np);
-        a1 = d.ws_i > 0.0 ? d.ws_i * h : 0.0;
+    if (ST == 3) {
+      const double h = iface ? row_dots(d, d.ri, j0, lc, u1) : 0.0;
+      if (mine) {
+        if (j < d.nvp) a1 = w_smooth(d, j) * lap_at(d, u1, j);
+        else a1 = d.ws_i > 0.0 ? d.ws_i * h : 0.0;
       }
     } else {
-      const double h = row_dot(d.rht, j, u1, d.np), v = row_dot(d.rvt, j, u2, d.np);
-      const bool m = masked(d, j);
-      a1 = d.ws_v * (m ? 0.0 : h);
-      a2 = d.ws_v * (m ? 0.0 : v);
-      if (j >= d.nvp && d.ws_i > 0.0 && d.ri.rp) {
-        ai = d.ws_i * row_dot(d.ri, j, u1, d.np);
-        has_i = true;
+      const double h = row_dots(d, d.rht, j0, lc, u1), v = row_dots(d, d.rvt, j0, lc, u2);
+      const bool ri = d.ws_i > 0.0 && d.ri.rp;
+      const double hi = ri && iface ? row_dots(d, d.ri, j0, lc, u1) : 0.0;
+      if (mine) {
+        const bool m = masked(d, j);
+        a1 = d.ws_v * (m ? 0.0 : h);
+        a2 = d.ws_v * (m ? 0.0 : v);
+        if (j >= d.nvp && ri) {
+          ai = d.ws_i * hi;
+          has_i = true;
+        }
       }
     }
-    if (lane == 0) {
+    if (mine) {
       double atu = g / bsc;
       atu = atu + a1 / bsc;
-      if (d.stype == 2) {
+      if (ST == 2) {
         atu = atu + a2 / bsc;
         if (has_i) atu = atu + ai / bsc;
       }
@@ -443,6 +558,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_adj_g(LsqrDev d) {
   adj_tail(d, ss, init);
 }
 
+template <int ST>
 __global__ void __launch_bounds__(kLsThreads) k_ls_fwd_g(LsqrDev d) {
   const int state = d.sc->state;
   if (state != kLsRun && state != kLsFinal) return;
@@ -458,23 +574,26 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_fwd_g(LsqrDev d) {
   double* u1 = d.u + d.nd;
   double* u2 = u1 + d.np;
   double* uD = damp_block(d);
+  const int lc = rows_log<ST>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
   if (run) {
     for (int i = warp; i < d.nd; i += nwarp) {
-      const double g = warp_dot(d.col, d.val, d.rp[i], d.rp[i + 1], d.v, d.np);
+      const double g = lc < 0 ? warp_dot(d.col, d.val, d.rp[i], d.rp[i + 1], d.v, d.np)
+                              : long_dot(d.col, d.val, d.rp[i], d.rp[i + 1], d.v, d.np);
       if (lane == 0) {
         const double un = g / asc - alpha * (d.u[i] / bsc);
         d.u[i] = un;
         ss += un * un;
       }
     }
-    for (int j = warp; j < d.np; j += nwarp) {
+    for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
+      const int j = j0 + lane / per;
       double s1, s2;
-      smooth_rows(d, d.v, j, &s1, &s2);
-      if (lane == 0) {
+      smooth_rows<ST>(d, d.v, j0, lc, j, &s1, &s2);
+      if ((lane & (per - 1)) == 0 && j < d.np) {
         const double a = s1 / asc - alpha * (u1[j] / bsc);
         u1[j] = a;
         ss += a * a;
-        if (d.stype == 2) {
+        if (ST == 2) {
           const double b = s2 / asc - alpha * (u2[j] / bsc);
           u2[j] = b;
           ss += b * b;
@@ -500,7 +619,7 @@ __global__ void k_spmv_rows(LsqrDev d, const double* __restrict__ x, double* __r
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarp = (gridDim.x * blockDim.x) >> 5;
   for (int i = warp; i < d.nd; i += nwarp) {
-    const double g = warp_dot(d.col, d.val, d.rp[i], d.rp[i + 1], x, d.np);
+    const double g = long_dot(d.col, d.val, d.rp[i], d.rp[i + 1], x, d.np);
     if (lane == 0) y[i] = g;
   }
 }
@@ -509,9 +628,11 @@ __global__ void k_spmv_cols(LsqrDev d, const double* __restrict__ x, double* __r
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarp = (gridDim.x * blockDim.x) >> 5;
-  for (int j = warp; j < d.np; j += nwarp) {
-    const double g = warp_dot(d.crow, d.cval, d.cp[j], d.cp[j + 1], x, d.nd);
-    if (lane == 0) y[j] = g;
+  const int lc = rows_log<1>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
+  for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
+    const double g = rows_dot(d.cp, d.crow, d.cval, j0, d.np, lc, x, d.nd, warp_span());
+    const int j = j0 + lane / per;
+    if ((lane & (per - 1)) == 0 && j < d.np) y[j] = g;
   }
 }
 
@@ -579,15 +700,18 @@ __global__ void k_csc_fill(const int* perm, const int* row_of, const double* val
 
 void lsqr_launch_init_u(const LsqrDev& d, int grid, cudaStream_t st) {
   if (d.stype == 1) k_ls_init_u<<<grid, kLsThreads, 0, st>>>(d);
-  else k_ls_init_u_g<<<grid, kLsThreads, 0, st>>>(d);
+  else if (d.stype == 2) k_ls_init_u_g<2><<<grid, kLsThreads, 0, st>>>(d);
+  else k_ls_init_u_g<3><<<grid, kLsThreads, 0, st>>>(d);
 }
 void lsqr_launch_adj(const LsqrDev& d, int grid, cudaStream_t st) {
   if (d.stype == 1) k_ls_adj<<<grid, kLsThreads, 0, st>>>(d);
-  else k_ls_adj_g<<<grid, kLsThreads, 0, st>>>(d);
+  else if (d.stype == 2) k_ls_adj_g<2><<<grid, kLsThreads, 0, st>>>(d);
+  else k_ls_adj_g<3><<<grid, kLsThreads, 0, st>>>(d);
 }
 void lsqr_launch_fwd(const LsqrDev& d, int grid, cudaStream_t st) {
   if (d.stype == 1) k_ls_fwd<<<grid, kLsThreads, 0, st>>>(d);
-  else k_ls_fwd_g<<<grid, kLsThreads, 0, st>>>(d);
+  else if (d.stype == 2) k_ls_fwd_g<2><<<grid, kLsThreads, 0, st>>>(d);
+  else k_ls_fwd_g<3><<<grid, kLsThreads, 0, st>>>(d);
 }
 void lsqr_launch_spmv(const LsqrDev& d, int transpose, const double* x, double* y, int grid,
                       cudaStream_t st) {
@@ -609,6 +733,7 @@ Lsqr::Lsqr(int device, cudaStream_t st) : device_(device), st_(st) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device_);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ls_adj, kLsThreads, 0);
   grid_ = std::max(1, nsm) * std::max(1, std::min(per_sm, 8));
+  grid3_ = std::max(1, nsm) * 6;   // smooth_type 3 (rows_log): fixed, the sums' order is by warp
   cudaMallocHost(&h_sc_, sizeof(LsqrScalars));
 }
 
@@ -713,7 +838,7 @@ std::string Lsqr::build_csc() {
   cp_.alloc((size_t)(np_ + 1) * 4);
   crow_.alloc((size_t)nnz * 4);
   cval_.alloc((size_t)nnz * 8);
-  part_.alloc((size_t)grid_ * 8);
+  part_.alloc((size_t)std::max(grid_, grid3_) * 8);
   sc_.alloc(sizeof(LsqrScalars));
   if (!cp_.p || !crow_.p || !cval_.p || !part_.p || !sc_.p) return "device allocation failed (CSC)";
   DevBuf row_of, iota, keys, perm, cnt, tmp;
@@ -899,6 +1024,7 @@ std::string Lsqr::solve(const LsqrParams& p, const double* residual, const doubl
   d.wd_i = p.wdv_iface;
   d.max_iter = p.max_iter;
   d.stype = p.smooth_type;
+  const int grid = d.stype == 3 ? grid3_ : grid_;
   if (d.stype != 1) {
     auto rows = [&](int k) {
       SpRows r;
@@ -925,16 +1051,16 @@ std::string Lsqr::solve(const LsqrParams& p, const double* residual, const doubl
   lsqr_launch_mask(d, gtg_.as<double>(), p.eps_min * 0.01, mask_.as<uint8_t>(), grid_, st_);
   LCK(cudaMemsetAsync(dm_.p, 0, (size_t)np_ * 8, st_));
   LCK(cudaMemsetAsync(sc_.p, 0, sizeof(LsqrScalars), st_));
-  lsqr_launch_init_u(d, grid_, st_);
-  lsqr_launch_adj(d, grid_, st_);
-  lsqr_launch_fwd(d, grid_, st_);
+  lsqr_launch_init_u(d, grid, st_);
+  lsqr_launch_adj(d, grid, st_);
+  lsqr_launch_fwd(d, grid, st_);
   launches += 4;
   LCK(cudaGetLastError());
   // the iteration loop: a graph of kIterPerGraph (adj, fwd) pairs
   LCK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < kIterPerGraph; ++k) {
-    lsqr_launch_adj(d, grid_, st_);
-    lsqr_launch_fwd(d, grid_, st_);
+    lsqr_launch_adj(d, grid, st_);
+    lsqr_launch_fwd(d, grid, st_);
   }
   LCK(cudaStreamEndCapture(st_, &r.graph));
   LCK(cudaGraphInstantiate(&r.exec, r.graph, 0));

@@ -136,7 +136,7 @@ class Lsqr {
   cudaStream_t st_;
   int nd_ = 0, np_ = 0, nvp_ = 0, if_start_ = 0, if_n_ = 0;
   long long nnz_ = 0;
-  int grid_ = 0;
+  int grid_ = 0, grid3_ = 0;   // blocks (smooth_type 1 and 2; 3)
   DevBuf rp_, col_, val_, cp_, crow_, cval_, nb_, mask_, res_, dms_, gtg_, u_, v_, w_, dm_,
       part_, sc_, x_, y_;
   // smoothing matrices: R_h, R_h^T, R_v, R_v^T, interface R_h
