@@ -209,6 +209,58 @@ enum { kIq = 0, kIx, kIt0, kIt1, kIb0, kIb1, kColN };
 typedef double CellMem[kCellN][kTraceThreads];
 typedef double ColMem[kColN][kTraceThreads];
 
+// A cell's loads: the columns' row ranges and the corners' gradients together.
+struct CellLoad {
+  int c, row, la, lb, ra, rb;
+  double2 a1, a2, a3, a4;
+};
+
+// (ix and ix + 1 are columns, iz and iz + 1 grid rows, from 1)
+__device__ __forceinline__ CellLoad load_cell(const TrRegion& r, const double2* G, int ix, int iz) {
+  CellLoad L;
+  L.c = ix - 1;
+  L.row = iz - 1;
+  const int br = L.row - r.z_lo;
+  const bool up = br >= 0 && br < r.H, dn = br + 1 >= 0 && br + 1 < r.H;
+  const int s0 = up ? br * r.pitch + L.c : 0, s1 = dn ? (br + 1) * r.pitch + L.c : 0;
+  L.la = r.r0[L.c];
+  L.lb = r.r1[L.c];
+  L.ra = r.r0[L.c + 1];
+  L.rb = r.r1[L.c + 1];
+  L.a1 = G[s0];
+  L.a2 = G[s0 + 1];
+  L.a3 = G[s1];
+  L.a4 = G[s1 + 1];
+  return L;
+}
+
+__device__ __forceinline__ void keep_cell(const TrRegion& r, const double2* G, CellMem& C,
+                                          CellLoad& L, double x, double z) {
+  const int t = threadIdx.x;
+  auto in = [](int k, int a, int b) { return k >= a && k <= b; };
+  const int mask = (in(L.row, L.la, L.lb) ? 1 : 0) | (in(L.row, L.ra, L.rb) ? 2 : 0) |
+                   (in(L.row + 1, L.la, L.lb) ? 4 : 0) | (in(L.row + 1, L.ra, L.rb) ? 8 : 0);
+  if (mask != 15) {
+    // a corner outside the region takes its column's nearest region node
+    auto other = [&](int bit, int k, int col, int a, int b, double2& g) {
+      if (mask & bit) return;
+      const int e = nearby_row(k, a, b);
+      g = e >= 0 ? G[(e - r.z_lo) * r.pitch + col] : make_double2(0.0, 0.0);
+    };
+    other(1, L.row, L.c, L.la, L.lb, L.a1);
+    other(2, L.row, L.c + 1, L.ra, L.rb, L.a2);
+    other(4, L.row + 1, L.c, L.la, L.lb, L.a3);
+    other(8, L.row + 1, L.c + 1, L.ra, L.rb, L.a4);
+  }
+  C[kCqx][t] = (double)L.c;
+  C[kCqz][t] = (double)L.row;
+  C[kCx][t] = x;
+  C[kCz][t] = z;
+  C[kCin][t] = (double)mask;
+  C[kCg1x][t] = L.a1.x; C[kCg2x][t] = L.a2.x; C[kCg3x][t] = L.a3.x; C[kCg4x][t] = L.a4.x;
+  C[kCg1z][t] = L.a1.y; C[kCg2z][t] = L.a2.y; C[kCg3z][t] = L.a3.y; C[kCg4z][t] = L.a4.y;
+}
+
 __device__ __noinline__ double2 enter_cell(const TrModel& M, const TrRegion& r, const double2* G,
                                            CellMem& C, double px, double pz) {
   const int t = threadIdx.x;
@@ -218,52 +270,23 @@ __device__ __noinline__ double2 enter_cell(const TrModel& M, const TrRegion& r, 
   iz = max(1, min(M.nz - 1, iz));
   const double x = gxc(M, ix), z = gzc(M, iz);
   if ((double)(ix - 1) != C[kCqx][t] || (double)(iz - 1) != C[kCqz][t]) {
-    C[kCqx][t] = (double)(ix - 1);
-    C[kCqz][t] = (double)(iz - 1);
-    C[kCx][t] = x;
-    C[kCz][t] = z;
-    // (ix and ix + 1 are columns, iz and iz + 1 grid rows): the columns' row
-    // ranges and the corners' gradients together
-    const int c = ix - 1, row = iz - 1, br = row - r.z_lo;
-    const bool up = br >= 0 && br < r.H, dn = br + 1 >= 0 && br + 1 < r.H;
-    const int s0 = up ? br * r.pitch + c : 0, s1 = dn ? (br + 1) * r.pitch + c : 0;
-    const int la = r.r0[c], lb = r.r1[c], ra = r.r0[c + 1], rb = r.r1[c + 1];
-    double2 a1 = G[s0], a2 = G[s0 + 1], a3 = G[s1], a4 = G[s1 + 1];
-    auto in = [](int k, int a, int b) { return k >= a && k <= b; };
-    if (!(in(row, la, lb) && in(row, ra, rb) && in(row + 1, la, lb) && in(row + 1, ra, rb))) {
-      // a corner outside the region takes its column's nearest region node
-      auto other = [&](int k, int col, int a, int b, double2& g) {
-        if (in(k, a, b)) return;
-        const int e = nearby_row(k, a, b);
-        g = e >= 0 ? G[(e - r.z_lo) * r.pitch + col] : make_double2(0.0, 0.0);
-      };
-      other(row, c, la, lb, a1);
-      other(row, c + 1, ra, rb, a2);
-      other(row + 1, c, la, lb, a3);
-      other(row + 1, c + 1, ra, rb, a4);
-    }
-    C[kCin][t] = (double)((in(row, la, lb) ? 1 : 0) | (in(row, ra, rb) ? 2 : 0) |
-                          (in(row + 1, la, lb) ? 4 : 0) | (in(row + 1, ra, rb) ? 8 : 0));
-    C[kCg1x][t] = a1.x; C[kCg2x][t] = a2.x; C[kCg3x][t] = a3.x; C[kCg4x][t] = a4.x;
-    C[kCg1z][t] = a1.y; C[kCg2z][t] = a2.y; C[kCg3z][t] = a3.y; C[kCg4z][t] = a4.y;
+    CellLoad L = load_cell(r, G, ix, iz);
+    keep_cell(r, G, C, L, x, z);
   }
   return make_double2(clamp01(quot(px - x, M.dx, M.rdx)), clamp01(quot(pz - z, M.dx, M.rdx)));
 }
 
-// rays2d.f90:825-894, in the ray's cell C (of the same region and field).
-__device__ __forceinline__ void grad_in(const TrModel& M, const TrRegion& r, const double2* G,
-                                        CellMem& C, double px, double pz, double& dtdx,
-                                        double& dtdz) {
+__device__ __forceinline__ bool in_cell(const TrModel& M, const CellMem& C, double px, double pz) {
   const int t = threadIdx.x;
-  double w1, w2;
-  if (inside((px - M.x0) * M.rdx, C[kCqx][t]) && inside((pz - 0.0) * M.rdx, C[kCqz][t])) {
-    w1 = share(px - C[kCx][t], M.dx, M.rdx);
-    w2 = share(pz - C[kCz][t], M.dx, M.rdx);
-  } else {
-    const double2 w = enter_cell(M, r, G, C, px, pz);
-    w1 = w.x;
-    w2 = w.y;
-  }
+  return inside((px - M.x0) * M.rdx, C[kCqx][t]) && inside((pz - 0.0) * M.rdx, C[kCqz][t]);
+}
+
+// rays2d.f90:825-894, in cell C with the point's shares w1, w2 of it.
+__device__ __forceinline__ void grad_of_cell(const TrModel& M, const TrRegion& r,
+                                             const double2* G, const CellMem& C, double px,
+                                             double pz, double w1, double w2, double& dtdx,
+                                             double& dtdz) {
+  const int t = threadIdx.x;
   double gx = (1.0 - w1) * (1.0 - w2) * C[kCg1x][t] + w1 * (1.0 - w2) * C[kCg2x][t] +
               (1.0 - w1) * w2 * C[kCg3x][t] + w1 * w2 * C[kCg4x][t];
   double gz = (1.0 - w1) * (1.0 - w2) * C[kCg1z][t] + w1 * (1.0 - w2) * C[kCg2z][t] +
@@ -295,6 +318,19 @@ __device__ __forceinline__ void grad_in(const TrModel& M, const TrRegion& r, con
   }
   dtdx = gx;
   dtdz = gz;
+}
+
+// The same, the point's cell to be made C if it is not.
+__device__ __forceinline__ void grad_in(const TrModel& M, const TrRegion& r, const double2* G,
+                                        CellMem& C, double px, double pz, double& dtdx,
+                                        double& dtdz) {
+  double2 w;
+  if (in_cell(M, C, px, pz))
+    w = make_double2(share(px - C[kCx][threadIdx.x], M.dx, M.rdx),
+                     share(pz - C[kCz][threadIdx.x], M.dx, M.rdx));
+  else
+    w = enter_cell(M, r, G, C, px, pz);
+  grad_of_cell(M, r, G, C, px, pz, w.x, w.y, dtdx, dtdz);
 }
 
 // The same with no cell to start from (C is left as the point's cell).
@@ -341,41 +377,67 @@ __device__ double iface_z(const TrModel& M, double px, int k) {
   return (1.0 - w) * z[ix - 1] + w * z[ix];
 }
 
-__device__ __noinline__ double2 enter_col(const TrModel& M, double px, const double* zt,
-                                          const double* zb, ColMem& C) {
-  const int t = threadIdx.x, nn = M.nx;
-  int ix = nn < 2 ? 0 : cell_of(px - M.xp0, M.dx, M.rdx) + 1;
-  if (ix < 1 || ix >= nn) {
-    ix = ix < 1 ? 0 : nn - 1;
-    return make_double2(zt[ix], zb[ix]);
-  }
-  const double x = M.xpos[ix - 1], t0 = zt[ix - 1], t1 = zt[ix], b0 = zb[ix - 1], b1 = zb[ix];
+// A column's loads.
+struct ColLoad {
+  int ix;                    // its first node, from 1; outside: 0 or nx
+  double x, t0, t1, b0, b1;
+};
+
+__device__ __forceinline__ ColLoad load_col(const TrModel& M, double px, const double* zt,
+                                            const double* zb) {
+  const int nn = M.nx;
+  ColLoad L;
+  L.ix = nn < 2 ? 0 : cell_of(px - M.xp0, M.dx, M.rdx) + 1;
+  L.ix = L.ix < 1 ? 0 : min(L.ix, nn);
+  const int a = L.ix < 1 ? 0 : L.ix - 1, b = L.ix < 1 || L.ix >= nn ? a : L.ix;
+  L.x = M.xpos[a];
+  L.t0 = zt[a];
+  L.t1 = zt[b];
+  L.b0 = zb[a];
+  L.b1 = zb[b];
+  return L;
+}
+
+// The column as C, and the interfaces at px (outside the nodes: the end's).
+__device__ __forceinline__ double2 keep_col(const TrModel& M, ColMem& C, const ColLoad& L,
+                                            double px) {
+  const int t = threadIdx.x;
+  if (L.ix < 1 || L.ix >= M.nx) return make_double2(L.t0, L.b0);
   // (the share's numerator is taken from the node's own x: inside's margin
   // holds where that is the grid's up to rounding)
-  const double q = (double)(ix - 1);
-  C[kIq][t] = fabs(x - (M.xp0 + q * M.dx)) < 1.0e-9 * M.dx ? q : -10.0;
-  C[kIx][t] = x;
-  C[kIt0][t] = t0;
-  C[kIt1][t] = t1;
-  C[kIb0][t] = b0;
-  C[kIb1][t] = b1;
-  const double w = clamp01(quot(px - x, M.dx, M.rdx));
-  return make_double2((1.0 - w) * t0 + w * t1, (1.0 - w) * b0 + w * b1);
+  const double q = (double)(L.ix - 1);
+  C[kIq][t] = fabs(L.x - (M.xp0 + q * M.dx)) < 1.0e-9 * M.dx ? q : -10.0;
+  C[kIx][t] = L.x;
+  C[kIt0][t] = L.t0;
+  C[kIt1][t] = L.t1;
+  C[kIb0][t] = L.b0;
+  C[kIb1][t] = L.b1;
+  const double w = clamp01(quot(px - L.x, M.dx, M.rdx));
+  return make_double2((1.0 - w) * L.t0 + w * L.t1, (1.0 - w) * L.b0 + w * L.b1);
+}
+
+__device__ __noinline__ double2 enter_col(const TrModel& M, double px, const double* zt,
+                                          const double* zb, ColMem& C) {
+  const ColLoad L = load_col(M, px, zt, zb);
+  return keep_col(M, C, L, px);
+}
+
+__device__ __forceinline__ bool in_col(const TrModel& M, const ColMem& C, double px) {
+  return inside((px - M.xp0) * M.rdx, C[kIq][threadIdx.x]);
+}
+__device__ __forceinline__ double2 pair_of_col(const TrModel& M, const ColMem& C, double px) {
+  const int t = threadIdx.x;
+  const double w = share(px - C[kIx][t], M.dx, M.rdx);
+  return make_double2((1.0 - w) * C[kIt0][t] + w * C[kIt1][t],
+                      (1.0 - w) * C[kIb0][t] + w * C[kIb1][t]);
 }
 
 // iface_z of a region's top and bottom interface at the same x.
 __device__ __forceinline__ void iface_pair(const TrModel& M, double px, const double* zt,
                                            const double* zb, ColMem& C, double& top, double& bot) {
-  const int t = threadIdx.x;
-  if (inside((px - M.xp0) * M.rdx, C[kIq][t])) {
-    const double w = share(px - C[kIx][t], M.dx, M.rdx);
-    top = (1.0 - w) * C[kIt0][t] + w * C[kIt1][t];
-    bot = (1.0 - w) * C[kIb0][t] + w * C[kIb1][t];
-  } else {
-    const double2 z = enter_col(M, px, zt, zb, C);
-    top = z.x;
-    bot = z.y;
-  }
+  const double2 z = in_col(M, C, px) ? pair_of_col(M, C, px) : enter_col(M, px, zt, zb, C);
+  top = z.x;
+  bot = z.y;
 }
 
 // rays2d.f90:1261-1306
@@ -538,10 +600,11 @@ struct Section {
   double x1, z1;           // first point
 };
 
-// A thread's cells: of the ray's point, of the predicted point, of anything else.
+// A thread's cells and columns: the last two that the ray's points and
+// predicted points were in, and those of anything else.
 struct TraceMem {
-  CellMem at, ahead, other;
-  ColMem col, ocol;
+  CellMem cell[2], other;
+  ColMem col[2], ocol;
 };
 
 __device__ __forceinline__ TraceMem& trace_mem() {
@@ -657,6 +720,7 @@ __device__ __forceinline__ void trace_ray(RayState<MODE>& R, bool active, double
   // still to be found), an invalid ray
   enum { kNext, kEnd, kExit, kInvalid, kHalve };
   double g0x = 0, g0z = 0, ppx = 0, ppz = 0, dl = 0;
+  int ci = 0, li = 0;          // the cell and the column used last
   // A point (px, pz) at or beyond interface k of the region ends the loop
   // (kExit), goes along the interface as a head wave or diffracted (kEnd: the
   // point is Xc, Zc), or may stay (kNext).  corrected: it is the corrector's
@@ -732,12 +796,46 @@ __device__ __forceinline__ void trace_ray(RayState<MODE>& R, bool active, double
     dl = dlmax;
     if (n == 2 && (on_bot || on_top)) dl = 10.0 * dlmax;
     double g1x, g1z;
-    grad_in(M, reg, G, C.at, Xp, Zp, g0x, g0z);
+    if (!in_cell(M, C.cell[ci], Xp, Zp)) ci ^= 1;
+    grad_in(M, reg, G, C.cell[ci], Xp, Zp, g0x, g0z);
     ppx = Xp - dl * g0x;
     ppz = Zp - dl * g0z;
-    // (the corrector's gradient at the predicted point, early: most steps need
-    // it, and its loads overlap the interface tests)
-    grad_in(M, reg, G, C.ahead, ppx, ppz, g1x, g1z);
+    // the corrector's gradient at the predicted point and the interfaces at its
+    // x: where one of them is not at hand, both are loaded (one wait a step for
+    // the warp: some lane enters a cell in nearly every step)
+    double zit, zib;
+    {
+      bool cm = !in_cell(M, C.cell[ci], ppx, ppz), lm = !in_col(M, C.col[li], ppx);
+      if (cm) {
+        ci ^= 1;
+        cm = !in_cell(M, C.cell[ci], ppx, ppz);
+      }
+      if (lm) {
+        li ^= 1;
+        lm = !in_col(M, C.col[li], ppx);
+      }
+      double2 wt, zz;
+      if (cm || lm) {
+        int ix = cell_of(ppx - M.x0, M.dx, M.rdx) + 1;
+        int iz = cell_of(ppz - 0.0, M.dx, M.rdx) + 1;
+        ix = max(1, min(M.nx - 1, ix));
+        iz = max(1, min(M.nz - 1, iz));
+        const double x = gxc(M, ix), z = gzc(M, iz);
+        CellLoad cl = load_cell(reg, G, ix, iz);
+        const ColLoad ll = load_col(M, ppx, ztop, zbot);
+        if (cm) keep_cell(reg, G, C.cell[ci], cl, x, z);
+        if (lm) zz = keep_col(M, C.col[li], ll, ppx);
+        wt = make_double2(clamp01(quot(ppx - x, M.dx, M.rdx)),
+                          clamp01(quot(ppz - z, M.dx, M.rdx)));
+      }
+      if (!cm)
+        wt = make_double2(share(ppx - C.cell[ci][kCx][threadIdx.x], M.dx, M.rdx),
+                          share(ppz - C.cell[ci][kCz][threadIdx.x], M.dx, M.rdx));
+      if (!lm) zz = pair_of_col(M, C.col[li], ppx);
+      zit = zz.x;
+      zib = zz.y;
+      grad_of_cell(M, reg, G, C.cell[ci], ppx, ppz, wt.x, wt.y, g1x, g1z);
+    }
     if (on_bot && ppz > Zp) ppz = 2.0 * Zp - ppz;
     if (on_top && ppz < Zp) ppz = 2.0 * Zp - ppz;
     if (n == 2 && start_direction != 0 && !refraction && seqnum != 1) {
@@ -761,8 +859,6 @@ __device__ __forceinline__ void trace_ray(RayState<MODE>& R, bool active, double
         }
       }
     }
-    double zit, zib;
-    iface_pair(M, ppx, ztop, zbot, C.col, zit, zib);
     int w = kStay;
     if (ppz <= zit) w = beyond(ppx, ppz, zit, iftop, on_top, false);
     if (w == kStay && ppz >= zib) w = beyond(ppx, ppz, zib, ifbot, on_bot, false);
@@ -772,7 +868,8 @@ __device__ __forceinline__ void trace_ray(RayState<MODE>& R, bool active, double
     ppz = Zp - dl * g0z;
     Xc = Xp - dl * (g0x + g1x) * 0.5;
     Zc = Zp - dl * (g0z + g1z) * 0.5;
-    iface_pair(M, Xc, ztop, zbot, C.col, zit, zib);
+    if (!in_col(M, C.col[li], Xc)) li ^= 1;
+    iface_pair(M, Xc, ztop, zbot, C.col[li], zit, zib);
     if (Zc <= zit) w = beyond(Xc, Zc, zit, iftop, on_top, true);
     if (w == kStay && Zc >= zib) w = beyond(Xc, Zc, zib, ifbot, on_bot, true);
     if (w != kStay) return settle(w, false);
@@ -867,7 +964,8 @@ __device__ __forceinline__ void trace_ray(RayState<MODE>& R, bool active, double
         rs.z1 = z_in;
         next_s = 4;
         flags_s = flags_k = -1;
-        C.at[kCqx][threadIdx.x] = C.ahead[kCqx][threadIdx.x] = C.col[kIq][threadIdx.x] = -10.0;
+        C.cell[0][kCqx][threadIdx.x] = C.cell[1][kCqx][threadIdx.x] = -10.0;
+        C.col[0][kIq][threadIdx.x] = C.col[1][kIq][threadIdx.x] = -10.0;
       }
       ++n;
       Xpp = Xp; Zpp = Zp;
