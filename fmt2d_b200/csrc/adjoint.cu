@@ -14,6 +14,7 @@
 // initialize_region_from_source2d (:2307-2411), the hand-off seeds of
 // sweep_region_from_interface2d (:1982-2304) and the PmP head-wave sweep
 // (src/inversion2d.f90:4294-4409).
+#include <math_constants.h>
 #include "adjoint.cuh"
 #define FMT_HD_LINK static
 #include "eik_eval.cuh"
@@ -697,27 +698,23 @@ __global__ void __launch_bounds__(256) k_adj_links(AdjField* fs, int nf) {
   }
 }
 
-// Nodes no link reads start the reverse sweep.
-__global__ void k_adj_front(AdjField* fs, int nf) {
+// The readers of slot s (the links that read its time, found among its
+// spread targets in their fixed order) with their weights, written at
+// roff[s]: the order the sweep sums them in.  Nodes no link reads start it.
+__global__ void k_adj_readers(AdjField* fs, int nf, AdjRead* rd) {
   AdjField& A = fs[blockIdx.y];
   const int ns = A.F.nslots();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
-  const int kind = A.link[s].kind;
-  if (kind == kAdjNone || A.cnt[s] != 0u) return;
-  A.fa[atomicAdd(&A.ctr[kAdjCtrFront], 1u)] = (unsigned)s;
-}
-
-// The readers of slot s (the links that read its time, found among its
-// spread targets in their fixed order) with their weights, written at
-// roff[s]: the order the sweep sums them in.
-__global__ void k_adj_readers(AdjField* fs, int nf, int* rk, double* rw) {
-  AdjField& A = fs[blockIdx.y];
-  const int ns = A.F.nslots();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns || A.rcnt[s] == 0u) return;
-  unsigned o = A.roff[s];
-  const unsigned end = o + A.rcnt[s];
+  const AdjLink& L = A.link[s];
+  if (L.kind == kAdjNone) return;   // (nothing reads it and it is not swept)
+  AdjNode N;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) N.t[j] = L.t[j];
+  N.ro = A.roff[s];
+  N.d = A.d[s];
+  const unsigned end = N.ro + A.rcnt[s];
+  unsigned o = N.ro;
   for (int q = 0; q < 16 && o < end; ++q) {
     const int k = ev::spread_target_at(A.F, s, q);
     if (k < 0) continue;
@@ -725,56 +722,99 @@ __global__ void k_adj_readers(AdjField* fs, int nf, int* rk, double* rw) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (K.t[j] == s && o < end) {
-        rk[o] = k;
-        rw[o] = K.wt[j];
+        rd[o].w = K.wt[j];
+        rd[o].k = k;
         ++o;
       }
   }
+  N.rc = o - N.ro;
+  A.node[s] = N;
+  if (A.rcnt[s] == 0u) A.fa[atomicAdd(&A.ctr[kAdjCtrFront], 1u)] = (unsigned)s;
 }
 
 // Reverse sweep of one field per block: a node is processed once every link
 // reading it has been (its count reaches zero), so each node is listed once
 // and the loop ends after at most one round per node.  lam[s] = d[s] + the
 // sum over its readers, in list order, of weight * lam[reader].
-__global__ void __launch_bounds__(1024) k_adj_sweep(AdjField* fs, int nf, const int* rk,
-                                                    const double* rw) {
-  AdjField& A = fs[blockIdx.x];
-  __shared__ unsigned n_in, n_out;
-  unsigned* fin = A.fa;
-  unsigned* fout = A.fb;
+// What bounds it: the latency of a round (thousands, one after the other).  A
+// node's chain is its list entry (shared memory, beyond kSweepCap in fa, fb),
+// one sector, its readers (contiguous) and their lam; the counts of the nodes
+// it reads go down meanwhile.  (With list, link, offsets and weights in arrays of
+// their own: 21.6 ms for 30 fields of 800,000 nodes, now 11.8.)
+constexpr unsigned kSweepCap = 4096;
+constexpr int kSweepThreads = 1024;
+__global__ void __launch_bounds__(kSweepThreads) k_adj_sweep(AdjField* fs, int nf,
+                                                             const AdjRead* rd) {
+  const AdjField& A = fs[blockIdx.x];
+  __shared__ unsigned list[2][kSweepCap];
+  __shared__ unsigned n_of[3];   // of this round, the next, the one after
+  unsigned* const far[2] = {A.fa, A.fb};
+  const AdjNode* node = A.node;
+  double* lam = A.lam;
+  unsigned* cnt = A.cnt;
+  const unsigned lane = threadIdx.x & 31u, full = 0xffffffffu;
+  const unsigned n0 = A.ctr[kAdjCtrFront];
+  for (unsigned i = threadIdx.x; i < min(n0, kSweepCap); i += kSweepThreads)
+    list[0][i] = far[0][i];
   if (threadIdx.x == 0) {
-    n_in = A.ctr[kAdjCtrFront];
-    n_out = 0;
+    n_of[0] = n0;
+    n_of[1] = n_of[2] = 0;
   }
   __syncthreads();
   unsigned done = 0, rounds = 0;
+  int cur = 0, a = 0;
   for (;;) {
-    const unsigned n = n_in;
+    const unsigned n = n_of[a];
     if (n == 0) break;
-    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
-      const int s = (int)fin[i];
-      double l = A.d[s];
-      const unsigned o = A.roff[s], c = A.rcnt[s];
-      for (unsigned e = 0; e < c; ++e) l += rw[o + e] * A.lam[rk[o + e]];
-      A.lam[s] = l;
-      const int* ts = A.link[s].t;   // a link is 8-byte aligned: plain int loads
+    const int b = a == 2 ? 0 : a + 1, c = b == 2 ? 0 : b + 1;
+    if (threadIdx.x == 0) n_of[c] = 0;
+    // (four lanes a node, one of the nodes it reads and of its readers each;
+    // whole warps)
+    for (unsigned k = threadIdx.x; k - lane < 4 * n; k += kSweepThreads) {
+      const unsigned i = k >> 2, sub = lane & 3u;
+      const bool on = i < n;
+      const int s = on ? (int)(i < kSweepCap ? list[cur][i] : far[cur][i]) : 0;
+      const AdjNode* N = node + s;
+      int t = -1;
+      unsigned ro = 0, rc = 0, left = 0;
+      double l = 0.0;
+      if (on) {
+        t = N->t[sub];
+        ro = N->ro;
+        rc = N->rc;
+        l = N->d;
+        if (t >= 0) left = atomicSub(cnt + t, 1u);
+      }
+      const unsigned most = __reduce_max_sync(full, rc);
+      for (unsigned e = 0; e < most; e += 4) {
+        AdjRead r;
+        r.w = 0.0;
+        double x = 0.0;
+        if (e + sub < rc) {
+          r = rd[ro + e + sub];
+          x = lam[r.k];
+        }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int t = ts[j];
-        if (t < 0) continue;
-        if (atomicSub(&A.cnt[t], 1u) == 1u) fout[atomicAdd(&n_out, 1u)] = (unsigned)t;
+        for (unsigned j = 0; j < 4; ++j) {
+          const double w = __shfl_sync(full, r.w, (lane & 28u) + j);
+          const double y = __shfl_sync(full, x, (lane & 28u) + j);
+          if (e + j < rc) l += w * y;
+        }
+      }
+      if (on && sub == 0) lam[s] = l;
+      const unsigned m = __ballot_sync(full, left == 1u);
+      unsigned p = 0;
+      if (lane == 0 && m) p = atomicAdd(&n_of[b], (unsigned)__popc(m));
+      p = __shfl_sync(full, p, 0) + __popc(m & ((1u << lane) - 1u));
+      if (left == 1u) {
+        if (p < kSweepCap) list[cur ^ 1][p] = (unsigned)t;
+        else far[cur ^ 1][p] = (unsigned)t;
       }
     }
-    __syncthreads();
     done += n;
     ++rounds;
-    if (threadIdx.x == 0) {
-      n_in = n_out;
-      n_out = 0;
-    }
-    unsigned* tmp = fin;
-    fin = fout;
-    fout = tmp;
+    cur ^= 1;
+    a = b;
     __syncthreads();
   }
   if (threadIdx.x == 0) {
@@ -837,34 +877,61 @@ __global__ void k_adj_handoff(AdjField* fs, const int* child, const int* parent,
   if (acc != 0.0) P.d[ps] += acc;
 }
 
-// The head-wave sweep reversed, one field per thread (k_headwave's order).
+// The head-wave sweep reversed (k_headwave's order), a block per field: its
+// chains run in one thread from shared memory, a batch of nodes at a time, with
+// the loads and stores spread over the block (a thread per field, its loads one
+// after the other, took 6 ms for 30 fields of 2001 nodes).
 // scratch: per field, nx doubles and 2*nx bytes.
-__global__ void k_adj_headwave(AdjField* fs, const int* which, int nsel, const int* hw_slot,
-                               const double* hw_v, const int* hw_vslot, double* const* pre,
-                               double dx_if, int nx, double* scratch) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsel) return;
+constexpr int kAdjHwBatch = 1024;
+__global__ void __launch_bounds__(256)
+    k_adj_headwave(AdjField* fs, const int* which, int nsel, const int* hw_slot,
+                   const double* hw_v, const int* hw_vslot, double* const* pre, double dx_if,
+                   int nx, double* scratch) {
+  const int q = blockIdx.x, tid = threadIdx.x;
   AdjField& A = fs[which[q]];
   double* th = scratch + (size_t)q * nx;
   uint8_t* fwd = reinterpret_cast<uint8_t*>(scratch + (size_t)nsel * nx) + (size_t)q * 2 * nx;
   uint8_t* bwd = fwd + nx;
   const double* p = pre[q];
-  for (int n = 0; n < nx; ++n) th[n] = hw_slot[n] >= 0 ? p[n] : kHugeD;
-  for (int n = 0; n < nx; ++n) { fwd[n] = 0; bwd[n] = 0; }
-  for (int n = 1; n < nx; ++n)
-    if (hw_v[n] > 0.0) {
-      const double c = th[n - 1] + dx_if / hw_v[n];
-      if (c < th[n]) fwd[n] = 1;
-      th[n] = fmin(th[n], c);
+  __shared__ double s_t[kAdjHwBatch], s_d[kAdjHwBatch], s_last;
+  __shared__ uint8_t s_f[kAdjHwBatch];
+  // the sweeps again: left to right (dir 1), back (-1); which nodes took the
+  // neighbour's time
+  auto sweep = [&](int dir, uint8_t* took) {
+    for (int b = 0; b < nx; b += kAdjHwBatch) {
+      const int m = min(kAdjHwBatch, nx - b);
+      for (int i = tid; i < m; i += blockDim.x) {
+        const int n = dir > 0 ? b + i : nx - 1 - (b + i);
+        s_t[i] = dir < 0 ? th[n] : hw_slot[n] >= 0 ? p[n] : kHugeD;
+        // (a node without a velocity keeps its time)
+        s_d[i] = hw_v[n] > 0.0 ? dx_if / hw_v[n] : CUDART_INF;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        double t = b ? s_last : s_t[0];
+        if (!b) s_f[0] = 0;
+#pragma unroll 4
+        for (int i = b ? 0 : 1; i < m; ++i) {
+          const double c = t + s_d[i], o = s_t[i];
+          s_f[i] = c < o;
+          t = fmin(o, c);
+          s_t[i] = t;
+        }
+        s_last = t;
+      }
+      __syncthreads();
+      for (int i = tid; i < m; i += blockDim.x) {
+        const int n = dir > 0 ? b + i : nx - 1 - (b + i);
+        th[n] = s_t[i];
+        took[n] = s_f[i];
+      }
+      __syncthreads();
     }
-  for (int n = nx - 2; n >= 0; --n)
-    if (hw_v[n] > 0.0) {
-      const double c = th[n + 1] + dx_if / hw_v[n];
-      if (c < th[n]) bwd[n] = 1;
-      th[n] = fmin(th[n], c);
-    }
+  };
+  sweep(1, fwd);
+  sweep(-1, bwd);
   // th now holds the sweep's values; reuse it for their adjoint
-  for (int n = 0; n < nx; ++n) {
+  for (int n = tid; n < nx; n += blockDim.x) {
     const int s = hw_slot[n];
     double g = 0.0;
     if (s >= 0 && th[n] < p[n] - 1.0e-10) {
@@ -873,21 +940,44 @@ __global__ void k_adj_headwave(AdjField* fs, const int* which, int nsel, const i
     }
     th[n] = g;
   }
-  for (int n = 0; n <= nx - 2; ++n)
-    if (bwd[n]) {
-      th[n + 1] += th[n];
-      const int vs = hw_vslot[n];
-      if (vs >= 0) A.gv[vs] += th[n] * (-dx_if / (hw_v[n] * hw_v[n]));
-      th[n] = 0.0;
+  __syncthreads();
+  // and its reversal: a node that took its neighbour's time hands its adjoint
+  // on (dir: to n + dir), and its velocity's slot gets a term
+  auto back = [&](int dir, const uint8_t* took) {
+    for (int b = 0; b < nx; b += kAdjHwBatch) {
+      const int m = min(kAdjHwBatch, nx - b);
+      for (int i = tid; i < m; i += blockDim.x) {
+        const int n = dir > 0 ? b + i : nx - 1 - (b + i);
+        s_t[i] = th[n];
+        s_f[i] = took[n];
+        s_d[i] = -dx_if / (hw_v[n] * hw_v[n]);
+      }
+      __syncthreads();
+      if (tid == 0) {
+        double carry = b ? s_last : 0.0;
+        bool has = b ? carry != 0.0 : false;
+        for (int i = 0; i < m; ++i) {
+          double t = s_t[i];
+          if (has) t += carry;
+          has = s_f[i] != 0;
+          if (has) {
+            const int n = dir > 0 ? b + i : nx - 1 - (b + i), vs = hw_vslot[n];
+            if (vs >= 0) A.gv[vs] += t * s_d[i];
+            carry = t;
+            t = 0.0;
+          }
+          s_t[i] = t;
+        }
+        s_last = has ? carry : 0.0;
+      }
+      __syncthreads();
+      for (int i = tid; i < m; i += blockDim.x) th[dir > 0 ? b + i : nx - 1 - (b + i)] = s_t[i];
+      __syncthreads();
     }
-  for (int n = nx - 1; n >= 1; --n)
-    if (fwd[n]) {
-      th[n - 1] += th[n];
-      const int vs = hw_vslot[n];
-      if (vs >= 0) A.gv[vs] += th[n] * (-dx_if / (hw_v[n] * hw_v[n]));
-      th[n] = 0.0;
-    }
-  for (int n = 0; n < nx; ++n)
+  };
+  back(1, bwd);
+  back(-1, fwd);
+  for (int n = tid; n < nx; n += blockDim.x)
     if (hw_slot[n] >= 0 && th[n] != 0.0) A.d[hw_slot[n]] += th[n];
 }
 
@@ -986,18 +1076,16 @@ void adj_links(AdjField* f, int nf, size_t max_slots, cudaStream_t st) {
   k_adj_links<<<grid, 256, 0, st>>>(f, nf);
 }
 
-void adj_readers(AdjField* f, int nf, size_t max_slots, int* rk, double* rw, cudaStream_t st) {
+void adj_readers(AdjField* f, int nf, size_t max_slots, AdjRead* rd, cudaStream_t st) {
   if (nf <= 0) return;
   const dim3 grid((unsigned)((max_slots + 255) / 256), nf);
-  k_adj_readers<<<grid, 256, 0, st>>>(f, nf, rk, rw);
+  k_adj_readers<<<grid, 256, 0, st>>>(f, nf, rd);
 }
 
-void adj_sweep(AdjField* f, int nf, size_t max_slots, const int* rk, const double* rw,
-               cudaStream_t st) {
+void adj_sweep(AdjField* f, int nf, size_t max_slots, const AdjRead* rd, cudaStream_t st) {
   if (nf <= 0) return;
   const dim3 grid((unsigned)((max_slots + 255) / 256), nf);
-  k_adj_front<<<grid, 256, 0, st>>>(f, nf);
-  k_adj_sweep<<<nf, 1024, 0, st>>>(f, nf, rk, rw);
+  k_adj_sweep<<<nf, kSweepThreads, 0, st>>>(f, nf, rd);
   k_adj_gv<<<grid, 256, 0, st>>>(f, nf);
 }
 
@@ -1011,7 +1099,7 @@ void adj_headwave(AdjField* f, const int* which, int nsel, const int* hw_slot, c
                   const int* hw_vslot, double* const* pre, double dx_if, int nx,
                   double* scratch, cudaStream_t st) {
   if (nsel <= 0) return;
-  k_adj_headwave<<<(nsel + 31) / 32, 32, 0, st>>>(f, which, nsel, hw_slot, hw_v, hw_vslot, pre,
+  k_adj_headwave<<<nsel, 256, 0, st>>>(f, which, nsel, hw_slot, hw_v, hw_vslot, pre,
                                                   dx_if, nx, scratch);
 }
 
@@ -1166,11 +1254,11 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
   DevBuf d_hwvslot;
   if (!(e = adj_put(d_hwvslot, hw_vslot_h_, stream_)).empty()) return e;
   // sources in chunks that fit in device memory
-  // per slot: link, counts, adjoint, direct term, velocity gradient, work
+  // per slot: link, node, counts, adjoint, direct term, velocity gradient, work
   // lists, reader count and offset, and up to 4 reader entries
-  constexpr size_t kPerSlot = sizeof(AdjLink) + 2 * sizeof(unsigned) + 3 * sizeof(double) +
+  constexpr size_t kPerSlot = sizeof(AdjLink) + sizeof(AdjNode) + 2 * sizeof(unsigned) + 3 * sizeof(double) +
                               2 * sizeof(unsigned) + 2 * sizeof(unsigned) +
-                              4 * (sizeof(int) + sizeof(double));
+                              4 * sizeof(AdjRead);
   size_t free_b = 0, total_b = 0;
   ACK(cudaMemGetInfo(&free_b, &total_b));
   const size_t budget = free_b / 2;
@@ -1206,11 +1294,12 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
     std::vector<size_t> off(nf + 1, 0);
     for (int i = 0; i < nf; ++i) off[i + 1] = off[i] + reg_[kTf[items[i].tf].reg].nslots;
     const size_t tot = off[nf];
-    DevBuf b_link, b_cnt, b_lam, b_d, b_gv, b_fa, b_fb, b_ctr, b_gz, b_rcnt, b_roff;
+    DevBuf b_link, b_node, b_cnt, b_lam, b_d, b_gv, b_fa, b_fb, b_ctr, b_gz, b_rcnt, b_roff;
     b_rcnt.alloc(tot * sizeof(unsigned));
     b_roff.alloc(tot * sizeof(unsigned));
     b_gz.alloc((size_t)nf * 3 * m_.nx * sizeof(double));
     b_link.alloc(tot * sizeof(AdjLink));
+    b_node.alloc(tot * sizeof(AdjNode));
     b_cnt.alloc(tot * sizeof(unsigned));
     b_lam.alloc(tot * sizeof(double));
     b_d.alloc(tot * sizeof(double));
@@ -1219,7 +1308,7 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
     b_fb.alloc(tot * sizeof(unsigned));
     b_ctr.alloc((size_t)nf * kAdjCtrN * sizeof(unsigned));
     if (!b_link.p || !b_cnt.p || !b_lam.p || !b_d.p || !b_gv.p || !b_fa.p || !b_fb.p || !b_ctr.p ||
-        !b_gz.p || !b_rcnt.p || !b_roff.p)
+        !b_gz.p || !b_rcnt.p || !b_roff.p || !b_node.p)
       return "device allocation failed (adjoint state)";
     ACK(cudaMemsetAsync(b_cnt.p, 0, tot * sizeof(unsigned), stream_));
     ACK(cudaMemsetAsync(b_lam.p, 0, tot * sizeof(double), stream_));
@@ -1233,6 +1322,7 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
       AdjField& A = hf[i];
       A.F = field_view(s, tf);
       A.link = b_link.as<AdjLink>() + off[i];
+      A.node = b_node.as<AdjNode>() + off[i];
       A.cnt = b_cnt.as<unsigned>() + off[i];
       A.lam = b_lam.as<double>() + off[i];
       A.d = b_d.as<double>() + off[i];
@@ -1389,12 +1479,11 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
                           stream_));
       ACK(cudaStreamSynchronize(stream_));
       const size_t nref = (size_t)last[0] + last[1];
-      DevBuf b_rk, b_rw;
-      b_rk.alloc(std::max<size_t>(nref, 1) * sizeof(int));
-      b_rw.alloc(std::max<size_t>(nref, 1) * sizeof(double));
-      if (!b_rk.p || !b_rw.p) return "device allocation failed (reader lists)";
-      adj_readers(dA + i0, i1 - i0, max_slots, b_rk.as<int>(), b_rw.as<double>(), stream_);
-      adj_sweep(dA + i0, i1 - i0, max_slots, b_rk.as<int>(), b_rw.as<double>(), stream_);
+      DevBuf b_rd;
+      b_rd.alloc(std::max<size_t>(nref, 1) * sizeof(AdjRead));
+      if (!b_rd.p) return "device allocation failed (reader lists)";
+      adj_readers(dA + i0, i1 - i0, max_slots, b_rd.as<AdjRead>(), stream_);
+      adj_sweep(dA + i0, i1 - i0, max_slots, b_rd.as<AdjRead>(), stream_);
       ACK(cudaGetLastError());
       ACK(cudaStreamSynchronize(stream_));
       i0 = i1;

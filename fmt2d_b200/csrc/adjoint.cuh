@@ -40,10 +40,24 @@ struct AdjLink {
   double wz[3];
 };
 
+// A node as the reverse sweep takes it, one sector: the nodes it reads, its
+// readers' place and number, its direct term.
+struct __align__(32) AdjNode {
+  int t[4];
+  unsigned ro, rc;
+  double d;
+};
+// A reader of a node: weight and slot.
+struct __align__(16) AdjRead {
+  double w;
+  int k, pad;
+};
+
 // One field's adjoint state.
 struct AdjField {
   Fld64 F;               // the solved field (frozen_slot set as the solve had it)
   AdjLink* link = nullptr;
+  AdjNode* node = nullptr;
   unsigned* cnt = nullptr;   // per slot: links reading its time that are not yet processed
   double* lam = nullptr;     // per slot: adjoint of the node's time
   double* d = nullptr;       // per slot: direct terms (picks, a child stage's hand-off)
@@ -81,13 +95,13 @@ enum {
 
 // Links of every slot of every field; counts each slot's readers.
 void adj_links(AdjField* f, int nf, size_t max_slots, cudaStream_t st);
-// Each node's readers (reader slot, link weight) at roff, in the fixed order
-// the sweep sums them (spread targets in order, then link entries in order).
-void adj_readers(AdjField* f, int nf, size_t max_slots, int* rk, double* rw, cudaStream_t st);
+// Each node's readers at roff, in the fixed order the sweep sums them (spread
+// targets in order, then link entries in order), the sweep's nodes (the direct
+// terms are final) and its first list: the nodes no link reads.
+void adj_readers(AdjField* f, int nf, size_t max_slots, AdjRead* rd, cudaStream_t st);
 // The reverse sweep (one block per field) over the reader lists and the
 // velocity gradient per slot.
-void adj_sweep(AdjField* f, int nf, size_t max_slots, const int* rk, const double* rw,
-               cudaStream_t st);
+void adj_sweep(AdjField* f, int nf, size_t max_slots, const AdjRead* rd, cudaStream_t st);
 // Hand-off terms: child field c's adjoint at its hand-off seeds is added to
 // its parent's direct terms (pairs child[k] -> parent[k], parent interface row
 // src_row of the child's seed descriptor).

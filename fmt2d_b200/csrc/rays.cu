@@ -13,7 +13,7 @@
 //
 // What bounds it: the latency of a ray's steps (up to 5000 a section, one
 // after the other), so the longest rays' chains (9000 steps of ~3600 cycles
-// alone in a warp, ~8000 in a full one) set the time.
+// alone in a warp, ~5500 in a full one) set the time.
 //  * The lanes of a warp step together and a warp takes as many rays as keep
 //    every warp resident (one where there are few picks), dealt strided, so
 //    that the neighbours on a receiver line, which are the same length, end up
@@ -24,13 +24,15 @@
 //    cell's gradients and the interface nodes around it in shared memory for
 //    the dozen steps a ray spends there (each lane reads its own lines: with a
 //    dozen warps on an SM the loads of every step took three times the step's
-//    own chain).
+//    own chain).  The last two cells and columns are kept, and a predicted point
+//    that enters a new one loads both at once: in a full warp some lane does in
+//    nearly every step, and all wait (45 -> 30 ms below).
 //  * The nine shorter steps of a ray at a head wave are tried by nine lanes at
 //    once instead of one after the other (7000 -> 800 cycles an event).
 //  * A ray caught in a cycle (a point it has been at before) is given up at
 //    once: it would go round until it runs out of points.
-// Times of 30276 picks on 2001 x 401 nodes: 150 -> 50 ms; 7870 picks on
-// 401 x 121, a third of them caught: 153 -> 19.5 ms.
+// Times of 30276 picks on 2001 x 401 nodes: 150 -> 30 ms; 7870 picks on
+// 401 x 121, a third of them caught: 153 -> 15 ms.
 //
 // A section's points are not stored: each segment is turned into its four
 // slowness-derivative contributions as soon as both ends are final (only the
@@ -200,11 +202,13 @@ __device__ __noinline__ int nearest_node(const TrModel& M, const TrRegion& r, do
 constexpr int kTraceThreads = 64;
 
 // Per thread of a block, in shared memory: a cell of a region's grid, the cell
-// between grid nodes a ray was in last, with its column and row from 0, its
-// corner node, the gradients at its corners (a corner outside the region takes
-// nearby_node's) and which of them are in the region (bits, corner 1 first); and the nodes of a region's top and bottom interface
-// around a column.
-enum { kCqx = 0, kCqz, kCx, kCz, kCg1x, kCg2x, kCg3x, kCg4x, kCg1z, kCg2z, kCg3z, kCg4z, kCin, kCellN };
+// between grid nodes a ray was in, with its column and row from 0, its corner
+// node, the gradients at its corners (a corner outside the region takes
+// nearby_node's) and which of them are in the region (bits, corner 1 first);
+// and the nodes of a region's top and bottom interface around a column.
+enum {
+  kCqx = 0, kCqz, kCx, kCz, kCg1x, kCg2x, kCg3x, kCg4x, kCg1z, kCg2z, kCg3z, kCg4z, kCin, kCellN
+};
 enum { kIq = 0, kIx, kIt0, kIt1, kIb0, kIb1, kColN };
 typedef double CellMem[kCellN][kTraceThreads];
 typedef double ColMem[kColN][kTraceThreads];
