@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstring>
 #include <cstdlib>
+#include <mutex>
 #include <thread>
 
 namespace fmt2d {
@@ -43,11 +44,12 @@ unsigned phase_fields(int mask) {
 void DevBuf::alloc(size_t n) {
   if (n <= bytes && p) return;
   free_();
-  if (cudaMalloc(&p, n < 16 ? 16 : n) != cudaSuccess) {
+  for (int tries = 0;; ++tries) {
+    if (cudaMalloc(&p, n < 16 ? 16 : n) == cudaSuccess) break;
     cudaGetLastError();   // the caller's to report: not the next launch check's
     p = nullptr;
     bytes = 0;
-    return;
+    if (tries || !Spare::reclaim()) return;
   }
   bytes = n;
 }
@@ -56,6 +58,52 @@ void DevBuf::free_() {
   if (p) cudaFree(p);
   p = nullptr;
   bytes = 0;
+}
+
+namespace {
+std::mutex g_spare_mu;
+std::vector<Spare*>& spares() {
+  static std::vector<Spare*>* v = new std::vector<Spare*>;   // (outlives every engine)
+  return *v;
+}
+}  // namespace
+
+void Spare::leave() {
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  auto& v = spares();
+  const auto it = std::find(v.begin(), v.end(), this);
+  if (it != v.end()) v.erase(it);
+}
+size_t Spare::bytes() const {
+  size_t n = 0;
+  for (const DevBuf* b : bufs_) n += b->bytes;
+  return n;
+}
+void Spare::release() {
+  for (DevBuf* b : bufs_) b->free_();
+}
+bool Spare::reclaim() {
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  bool any = false;
+  for (Spare* s : spares())
+    if (!s->busy_ && s->bytes() > 0) {
+      s->release();
+      any = true;
+    }
+  return any;
+}
+Spare::Use::Use(Spare& s, int share) : s_(s), share_(share) {
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  s_.busy_ = true;
+  auto& v = spares();
+  if (std::find(v.begin(), v.end(), &s_) == v.end()) v.push_back(&s_);
+}
+Spare::Use::~Use() {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) total_b = 0;
+  std::lock_guard<std::mutex> lock(g_spare_mu);
+  if (s_.bytes() > total_b / share_) s_.release();
+  s_.busy_ = false;
 }
 
 namespace {
@@ -267,7 +315,6 @@ std::string Engine::forward(const double* sx, int nsrc, int phase_mask) {
       F.solved = false;
       if (!(need & (1u << tf))) continue;
       const DevRegionStore& D = reg_[kTf[tf].reg];
-      if (F.T.bytes < D.nslots * 8) rowspace_.release();
       F.T.alloc(D.nslots * 8);
       F.G.alloc(D.nslots * 16);
       F.Gout.alloc(D.nslots * 16);

@@ -48,6 +48,35 @@ struct DevBuf {
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Buffers an engine keeps from one call for the next.  When a call is over
+// (Use's end) they stay only if they take no more than a share of the device's
+// memory, and while no call uses them any allocation of the library that finds
+// no memory takes them back (reclaim, from any engine and thread).
+class Spare {
+ public:
+  Spare() = default;
+  Spare(const Spare&) = delete;
+  Spare& operator=(const Spare&) = delete;
+  size_t bytes() const;
+  class Use {
+   public:
+    Use(Spare& s, int share);
+    ~Use();
+   private:
+    Spare& s_;
+    int share_;
+  };
+  static bool reclaim();   // whether anything was freed
+
+ protected:
+  std::vector<DevBuf*> bufs_;
+  void leave();            // before the buffers go
+
+ private:
+  void release();
+  bool busy_ = false;
+};
+
 // Static device data of one region (slot layout of model.h).
 struct DevRegionStore {
   DevBuf code, vel64, izc, iface_x, iface_z, r0, r1, slot_of_node;
@@ -197,14 +226,18 @@ class Engine {
       d_tcalc_, d_valid_, d_cnt_, d_off_, d_rowptr_, d_tmp_, d_col_, d_val_, d_sft_, d_sfjobs_,
       d_entry_;
   // Frechet rows' workspace: sort keys and values, the pool of the rays'
-  // entries (the sort's second buffers later), its chunks' owners and counter.
-  // Kept while it is a small part of the device's memory (trace), given back
-  // when the time fields grow (forward)
-  struct RowSpace {
+  // entries (the sort's second buffers later), its chunks' owners and counter
+  struct RowSpace : Spare {
     DevBuf keys, vals, ids, pvals, owner, used;
-    size_t bytes() const { return keys.bytes + vals.bytes + ids.bytes + pvals.bytes + owner.bytes; }
-    void release();
+    RowSpace() { bufs_ = {&keys, &vals, &ids, &pvals, &owner, &used}; }
+    ~RowSpace() { leave(); }
   } rowspace_;
+  // The adjoint's state of a chunk of sources (misfit_gradient)
+  struct AdjSpace : Spare {
+    DevBuf link, node, cnt, lam, d, gv, fa, fb, rcnt, roff, rd;
+    AdjSpace() { bufs_ = {&link, &node, &cnt, &lam, &d, &gv, &fa, &fb, &rcnt, &roff, &rd}; }
+    ~AdjSpace() { leave(); }
+  } adjspace_;
   int npick_ = -1, rows_ = 0;
   long long nnz_ = 0;
   double trace_ms_ = 0.0;

@@ -105,10 +105,6 @@ std::string Engine::upload_trace_tables() {
   return std::string();
 }
 
-void Engine::RowSpace::release() {
-  for (DevBuf* b : {&keys, &vals, &ids, &pvals, &owner, &used}) b->free_();
-}
-
 std::string Engine::trace(const int* src, const int* phase, const double* rx, const double* rz,
                           int npick, double* t_calc, int* valid, long long* nnz, bool rows) {
   cudaSetDevice(device_);
@@ -195,6 +191,7 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
     // twice (four a cell); where that is too little, or memory is short, the
     // rays that count their entries are traced again into one of the right size
     RowSpace& W = rowspace_;
+    const Spare::Use use(W, 16);
     size_t chunks = 0;
     TrPool pool;
     auto set_pool = [&](size_t n) {
@@ -265,14 +262,6 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
     TCK(cudaMemcpyAsync(&used, W.used.p, sizeof(used), cudaMemcpyDeviceToHost, stream_));
     TCK(cudaStreamSynchronize(stream_));
     if (total >= 0x7fffffffull) return "too many Frechet contributions for 32-bit CSR";
-    struct Keep {   // the workspace stays only while it is small, whatever the way out
-      RowSpace& w;
-      ~Keep() {
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || w.bytes() > total_b / 16)
-          w.release();
-      }
-    } keep{W};
     if (used > pool.nchunks) {
       if (!set_pool((size_t)total / kTrChunk + npick)) return "device allocation failed (Frechet)";
       TCK(cudaMemsetAsync(W.used.p, 0, sizeof(unsigned), stream_));

@@ -52,3 +52,33 @@ def test_rows_with_little_memory(count, short):
     assert n2 == n + (1 if short else 0)   # the second trace
     assert nnz2 == nnz and t.tobytes() == t2.tobytes() and np.array_equal(v, v2)
     assert all(a.tobytes() == b.tobytes() for a, b in zip(r, r2))
+
+
+def test_kept_buffers_are_given_back():
+    """What a trace with rows and a gradient keep for the next call goes back
+    when another engine finds no memory, and both engines' results stay."""
+    import torch
+    from fmt2d_b200.api import Fmt2d
+    m = synth.small_model(phases=(1, 3), seed=9)
+    pk = m.picks[np.arange(6000) % len(m.picks)]
+    args = (pk[:, 0].astype(np.int32), pk[:, 1].astype(np.int32), pk[:, 2].copy(), pk[:, 3].copy())
+
+    def results(g):
+        t, v, _ = g.trace(*args)
+        rows = [a.copy() for a in g.frechet_rows(index_base=0)]
+        grad = g.misfit_gradient(*args, np.where(v, t + 0.01, -1.0), 0.04, want=("slow",))
+        return [t, v, *rows, grad["grad_slow"]]
+
+    a = Fmt2d(0).upload(m)
+    a.forward(m.obs_x, (1, 3))
+    want = results(a)
+    b = Fmt2d(0).upload(m)
+    free, _ = torch.cuda.mem_get_info()
+    fill = torch.empty(max(0, free - (8 << 20)), dtype=torch.uint8, device="cuda")
+    b.forward(m.obs_x, (1, 3))   # its fields do not fit beside what a has kept
+    del fill
+    torch.cuda.empty_cache()
+    for g in (b, a):
+        for x, y in zip(want, results(g)):
+            assert x.tobytes() == y.tobytes()
+        g.close()
