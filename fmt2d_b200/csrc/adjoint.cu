@@ -31,115 +31,139 @@ using ev::RNb;
 // ---------------------------------------------------------------- duals
 constexpr int kND = 8;   // independent inputs of one candidate
 
-struct Dn {
+template <int N>
+struct DualN {
   double v;
-  double d[kND];
+  double d[N];
 };
+typedef DualN<kND> Dn;
 
-__device__ inline Dn dconst(double v) {
-  Dn r;
+template <int N = kND>
+__device__ inline DualN<N> dconst(double v) {
+  DualN<N> r;
   r.v = v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = 0.0;
+  for (int k = 0; k < N; ++k) r.d[k] = 0.0;
   return r;
 }
-__device__ inline Dn dvar(double v, int k) {
-  Dn r = dconst(v);
+template <int N = kND>
+__device__ inline DualN<N> dvar(double v, int k) {
+  DualN<N> r = dconst<N>(v);
   if (k >= 0) r.d[k] = 1.0;
   return r;
 }
-__device__ inline Dn operator+(const Dn& a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator+(const DualN<N>& a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a.v + b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = a.d[k] + b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] + b.d[k];
   return r;
 }
-__device__ inline Dn operator-(const Dn& a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator-(const DualN<N>& a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a.v - b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = a.d[k] - b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] - b.d[k];
   return r;
 }
-__device__ inline Dn operator-(const Dn& a) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator-(const DualN<N>& a) {
+  DualN<N> r;
   r.v = -a.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = -a.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = -a.d[k];
   return r;
 }
-__device__ inline Dn operator*(const Dn& a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator*(const DualN<N>& a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a.v * b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
   return r;
 }
-__device__ inline Dn operator/(const Dn& a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator/(const DualN<N>& a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a.v / b.v;
   const double ib = 1.0 / b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * ib;
+  for (int k = 0; k < N; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * ib;
   return r;
 }
-__device__ inline Dn operator*(double a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator*(double a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a * b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = a * b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a * b.d[k];
   return r;
 }
-__device__ inline Dn operator*(const Dn& a, double b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator*(const DualN<N>& a, double b) {
+  DualN<N> r;
   r.v = a.v * b;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = a.d[k] * b;
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b;
   return r;
 }
-__device__ inline Dn operator/(const Dn& a, double b) {
-  Dn r;
+// (b > 0; a derivative that is zero, as most are, stays: the division of a zero
+// leaves the compiler's short one, about 500 cycles for the whole warp)
+template <int N>
+__device__ inline DualN<N> operator/(const DualN<N>& a, double b) {
+  DualN<N> r;
   r.v = a.v / b;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = a.d[k] / b;
+  for (int k = 0; k < N; ++k) {
+    double n = a.d[k];
+    if (n != 0.0) n = n / b;
+    r.d[k] = n;
+  }
   return r;
 }
-__device__ inline Dn operator/(double a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator/(double a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a / b.v;
   const double f = -r.v / b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = f * b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = f * b.d[k];
   return r;
 }
-__device__ inline Dn operator+(double a, const Dn& b) {
-  Dn r = b;
+template <int N>
+__device__ inline DualN<N> operator+(double a, const DualN<N>& b) {
+  DualN<N> r = b;
   r.v = a + b.v;
   return r;
 }
-__device__ inline Dn operator-(double a, const Dn& b) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> operator-(double a, const DualN<N>& b) {
+  DualN<N> r;
   r.v = a - b.v;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = -b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = -b.d[k];
   return r;
 }
-__device__ inline Dn operator-(const Dn& a, double b) {
-  Dn r = a;
+template <int N>
+__device__ inline DualN<N> operator-(const DualN<N>& a, double b) {
+  DualN<N> r = a;
   r.v = a.v - b;
   return r;
 }
-__device__ inline Dn dsqrt(const Dn& a) {
-  Dn r;
+template <int N>
+__device__ inline DualN<N> dsqrt(const DualN<N>& a) {
+  DualN<N> r;
   r.v = sqrt(a.v);
   const double f = r.v > 0.0 ? 0.5 / r.v : 0.0;
 #pragma unroll
-  for (int k = 0; k < kND; ++k) r.d[k] = f * a.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = f * a.d[k];
   return r;
 }
 // fmax(a, b) for the non-NaN operands the stencil has: the larger; a on ties
-__device__ inline Dn dmax(const Dn& a, const Dn& b) { return b.v > a.v ? b : a; }
+template <int N>
+__device__ inline DualN<N> dmax(const DualN<N>& a, const DualN<N>& b) { return b.v > a.v ? b : a; }
 
 // Where each dual input comes from: a same-field time (tslot), a slot
 // velocity (vslot) or the parent field's time (xslot).
@@ -152,43 +176,6 @@ struct Inputs {
 };
 
 // ------------------------------------------------- candidate re-derivation
-// A direct neighbour in dual form (rnb4's values for one direction).
-struct DNb {
-  bool dirx, second;
-  Dn T, T2, d2;
-};
-
-// regular_update2d for one or two neighbours (ev::reg_cand's expressions).
-__device__ bool reg_dual(const DNb* p, const DNb* q, Dn& out) {
-  Dn a = dconst(0.0), b = dconst(0.0), c = dconst(0.0), tmax = dconst(0.0);
-  for (int k = 0; k < 2; ++k) {
-    const DNb* n = k == 0 ? p : q;
-    if (!n) continue;
-    tmax = dmax(tmax, n->T);
-    if (n->second) {
-      const Dn tx = n->T, t2x = n->T2;
-      a = a + 2.25 * n->d2;
-      b = b + (-6.0 * tx + 1.5 * t2x) * n->d2;
-      c = c + (4.0 * tx * tx - 2.0 * tx * t2x + 0.25 * t2x * t2x) * n->d2;
-    } else {
-      const Dn tx = n->T;
-      a = a + n->d2;
-      b = b + (-2.0 * tx) * n->d2;
-      c = c + (tx * tx) * n->d2;
-    }
-  }
-  c = c - 1.0;
-  if (fabs(a.v) < ev::kTinyD) return false;
-  Dn det = b * b - 4.0 * a * c;
-  if (det.v < 0.0) {
-    if (0.5 * sqrt(fabs(det.v)) / fabs(a.v) < 1.0e20) det = dconst(0.0);
-    else return false;
-  }
-  const Dn t1 = 0.5 * (-b + dsqrt(det)) / a;
-  out = dmax(t1, tmax);
-  return true;
-}
-
 // time_from_1_node2d (ev::from_1): a copy when the member is within
 // 0.01*tolerance, else the member's time plus the straight ray.  Depths az
 // (the member) and zu (the node) are inputs: interface nodes move with their
@@ -399,30 +386,70 @@ __device__ int iface_members_s(const Fld64& F, int side, int col, uint32_t code,
   return nm;
 }
 
-// The direct neighbour `dir` of grid node (r, c) (rnb4's order L, R, U, D)
-// in dual form; inputs are appended from index k.
-__device__ DNb dual_nb(const Fld64& F, const RNb& n, int r, int c, int dir, const Dn& vu,
-                       int& k, Inputs& in) {
-  const int dr[4] = {0, 0, -1, 1}, dc[4] = {-1, 1, 0, 0};
-  const int s1 = (r + dr[dir]) * F.pitch + (c + dc[dir]);
-  const int s2 = (r + 2 * dr[dir]) * F.pitch + (c + 2 * dc[dir]);
-  DNb o;
-  o.dirx = n.dirx;
-  o.second = n.second;
-  in.tslot[k] = s1;
-  o.T = dvar(n.T, k++);
-  if (n.second) {
-    in.tslot[k] = s2;
-    o.T2 = dvar(n.T2, k++);
-  } else {
-    o.T2 = dconst(0.0);
+// The link of slot s whose winner is regular_update2d's (ev::reg_cand's
+// expressions), with the inputs at fixed places: 0 the node's velocity; 1, 2, 3
+// the horizontal neighbour's time, the one behind's and its velocity; 4, 5, 6 the
+// vertical ones.  (Nearly all nodes are such: with places counted up as inputs
+// are met, the duals lived in local memory, and k_adj_links took 19 ms for 60
+// fields of 800,000 nodes; now 9.6.)
+__device__ __forceinline__ void regular_link(const Fld64& F, int s, double vu, const RNb* nb,
+                                             const Win& w, double Ts, AdjLink& L) {
+  typedef DualN<7> D;
+  const bool hx = w.x >= 0, hz = w.z >= 0;
+  const RNb X = w.x == 1 ? nb[1] : nb[0], Z = w.z == 3 ? nb[3] : nb[2];
+  const int ox = w.x == 1 ? 1 : -1, oz = w.z == 3 ? F.pitch : -F.pitch;
+  const D vud = dvar<7>(vu, 0);
+  D a = dconst<7>(0.0), b = dconst<7>(0.0), c = dconst<7>(0.0), tmax = dconst<7>(0.0);
+  auto add = [&](const RNb& n, int s1, int k0) {
+    const D tx = dvar<7>(n.T, k0), v1 = dvar<7>(FMT_RO(F.vel + s1), k0 + 2);
+    const D dd = 0.5 * (vud + v1) / F.dx, d2 = dd * dd;
+    tmax = dmax(tmax, tx);
+    if (n.second) {
+      const D t2x = dvar<7>(n.T2, k0 + 1);
+      a = a + 2.25 * d2;
+      b = b + (-6.0 * tx + 1.5 * t2x) * d2;
+      c = c + (4.0 * tx * tx - 2.0 * tx * t2x + 0.25 * t2x * t2x) * d2;
+    } else {
+      a = a + d2;
+      b = b + (-2.0 * tx) * d2;
+      c = c + (tx * tx) * d2;
+    }
+  };
+  if (hx) add(X, s + ox, 1);
+  if (hz) add(Z, s + oz, 4);
+  c = c - 1.0;
+  bool ok = !(fabs(a.v) < ev::kTinyD);
+  D det = b * b - 4.0 * a * c;
+  if (det.v < 0.0) {
+    if (0.5 * sqrt(fabs(det.v)) / fabs(a.v) < 1.0e20) det = dconst<7>(0.0);
+    else ok = false;
   }
-  in.vslot[k] = s1;
-  const Dn v1 = dvar(FMT_RO(F.vel + s1), k++);
-  const Dn velx = 0.5 * (vu + v1);
-  const Dn dd = velx / F.dx;
-  o.d2 = dd * dd;
-  return o;
+  const D t1 = 0.5 * (-b + dsqrt(det)) / a;
+  const D val = dmax(t1, tmax);
+  if (!ok || __double_as_longlong(val.v) != __double_as_longlong(Ts)) {
+    L.kind = kAdjMismatch;
+    return;
+  }
+  L.kind = kAdjRegular;
+  int nt = 0, nv = 1;
+  L.v[0] = s;
+  L.wv[0] = val.d[0];
+  auto put = [](int& n, int* slot, double* wt, int t, double d) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n == j) { slot[j] = t; wt[j] = d; }
+    ++n;
+  };
+  if (hx) {
+    put(nt, L.t, L.wt, s + ox, val.d[1]);
+    if (X.second) put(nt, L.t, L.wt, s + 2 * ox, val.d[2]);
+    put(nv, L.v, L.wv, s + ox, val.d[3]);
+  }
+  if (hz) {
+    put(nt, L.t, L.wt, s + oz, val.d[4]);
+    if (Z.second) put(nt, L.t, L.wt, s + 2 * oz, val.d[5]);
+    put(nv, L.v, L.wv, s + oz, val.d[6]);
+  }
 }
 
 // Seed of slot s in dual form (k_init_source, k_seed_iface).
@@ -596,19 +623,8 @@ __device__ bool derive(const AdjField& A, int s, AdjLink& L) {
   if (seeded) {
     ok = seed_dual(A, s, row, col, val, in, kind);
   } else if (w.kind == kAdjRegular) {
-    int k = 0;
-    in.vslot[k] = s;
-    const Dn vud = dvar(vu, k++);
-    DNb dx_, dz_;
-    const DNb* P = nullptr;
-    const DNb* Q = nullptr;
-    if (w.x >= 0) { dx_ = dual_nb(F, nb[w.x], row, col, w.x, vud, k, in); P = &dx_; }
-    if (w.z >= 0) {
-      dz_ = dual_nb(F, nb[w.z], row, col, w.z, vud, k, in);
-      if (P) Q = &dz_; else P = &dz_;
-    }
-    ok = reg_dual(P, Q, val);
-    kind = kAdjRegular;
+    regular_link(F, s, vu, nb, w, Ts, L);
+    return true;
   } else if (w.kind == kAdjRay || w.kind == kAdjPlane) {
     Mem m[6];
     int ms[6];
@@ -683,8 +699,14 @@ __global__ void __launch_bounds__(256) k_adj_links(AdjField* fs, int nf) {
         if (t < 0) continue;
         atomicAdd(&A.cnt[t], 1u);
         // the reverse sweep finds a node's readers among its spread targets
+        // (a grid node's grid targets are its 3x3 block and the second neighbours
+        // along the axes)
+        const int pitch = A.F.pitch, rs = s / pitch, rt = t / pitch;
+        const int dr = abs(rs - rt), dc = abs((s - rs * pitch) - (t - rt * pitch));
         bool listed = false;
-        for (int q = 0; q < 16; ++q) listed = listed || ev::spread_target_at(A.F, t, q) == s;
+        if (rs < A.F.H && rt < A.F.H) listed = dr + dc > 0 && (max(dr, dc) == 1 || dr + dc == 2);
+        else
+          for (int q = 0; q < 16; ++q) listed = listed || ev::spread_target_at(A.F, t, q) == s;
         if (!listed) atomicAdd(&n_unl, 1u);
       }
     }
