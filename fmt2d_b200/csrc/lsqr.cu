@@ -216,12 +216,14 @@ __device__ __forceinline__ double rows_dot(const int* __restrict__ rp,
 // of smooth_type 3, the inversion's usual one, keeps a warp a row and the order
 // of every sum (-1): the line search's rays are traced in its solution, and a
 // ray can turn on the last bit.
+__host__ __device__ inline int rows_log(int n, int nwarp) {
+  int lc = 0;
+  while (lc < 5 && (n >> (lc + 1)) >= nwarp) ++lc;
+  return lc;
+}
 template <int ST>
 __device__ __forceinline__ int rows_log(const LsqrDev& d, int nwarp) {
-  if (ST == 3) return -1;
-  int lc = 0;
-  while (lc < 5 && (d.np >> (lc + 1)) >= nwarp) ++lc;
-  return lc;
+  return ST == 3 ? -1 : rows_log(d.np, nwarp);
 }
 
 __device__ __forceinline__ double* warp_span() {
@@ -362,11 +364,13 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_adj(LsqrDev d) {
   const double* uL = d.u + d.nd;
   const double* uD = d.u + d.nd + d.np;
   double ss = 0.0;
-  const int lc = rows_log<1>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
-  for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
-    const double g = rows_dot(d.cp, d.crow, d.cval, j0, d.np, lc, d.u, d.nd, warp_span());
-    const int j = j0 + lane / per;
-    if ((lane & (per - 1)) == 0 && j < d.np) {
+  const int per = 32 >> d.task_log;
+  for (int t = warp; t < d.ntask; t += nwarp) {
+    const int2 T = d.task[t];
+    const double g = rows_dot(d.cp, d.crow, d.cval, T.x, T.x + T.y, d.task_log, d.u, d.nd,
+                              warp_span());
+    const int j = T.x + lane / per;
+    if ((lane & (per - 1)) == 0 && j < T.x + T.y) {
       double atu = g / bsc;
       atu = atu + (w_smooth(d, j) * lap_at(d, uL, j)) / bsc;
       atu = atu + (w_damp(d, j) * uD[j]) / bsc;
@@ -500,7 +504,7 @@ __global__ void __launch_bounds__(kLsThreads) k_ls_init_u_g(LsqrDev d) {
 }
 
 template <int ST>
-__global__ void __launch_bounds__(kLsThreads) k_ls_adj_g(LsqrDev d) {
+__global__ void __launch_bounds__(kLsThreads, ST == 2 ? 4 : 1) k_ls_adj_g(LsqrDev d) {
   const int state = d.sc->state;
   if (state != kLsInit && state != kLsRun) return;
   const bool init = state == kLsInit;
@@ -628,11 +632,13 @@ __global__ void k_spmv_cols(LsqrDev d, const double* __restrict__ x, double* __r
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarp = (gridDim.x * blockDim.x) >> 5;
-  const int lc = rows_log<1>(d, nwarp), rows = lc < 0 ? 1 : 1 << lc, per = 32 / rows;
-  for (int j0 = warp * rows; j0 < d.np; j0 += nwarp * rows) {
-    const double g = rows_dot(d.cp, d.crow, d.cval, j0, d.np, lc, x, d.nd, warp_span());
-    const int j = j0 + lane / per;
-    if ((lane & (per - 1)) == 0 && j < d.np) y[j] = g;
+  const int per = 32 >> d.task_log;
+  for (int t = warp; t < d.ntask; t += nwarp) {
+    const int2 T = d.task[t];
+    const double g = rows_dot(d.cp, d.crow, d.cval, T.x, T.x + T.y, d.task_log, x, d.nd,
+                              warp_span());
+    const int j = T.x + lane / per;
+    if ((lane & (per - 1)) == 0 && j < T.x + T.y) y[j] = g;
   }
 }
 
@@ -694,6 +700,26 @@ __global__ void k_csc_fill(const int* perm, const int* row_of, const double* val
     crow[k] = row_of[p];
     cval[k] = val[p];
   }
+}
+
+// Runs of columns for a warp each: within every 2^lc columns, a new run where
+// the entries would pass kTaskEntries (columns at the sources hold those of
+// thousands of rays: a warp with 32 of them would end long after the others).
+// Writes the runs of block b at task + first[b], or only counts them.
+constexpr int kTaskEntries = 4 * kSpan;
+__global__ void k_tasks(const int* cp, int np, int lc, int nblock, int* count, const int* first,
+                        int2* task) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nblock) return;
+  const int j1 = min(np, (b + 1) << lc);
+  int n = 0, j0 = b << lc;
+  for (int j = j0 + 1; j <= j1; ++j)
+    if (j == j1 || cp[j + 1] - cp[j0] > kTaskEntries) {
+      if (task) task[first[b] + n] = make_int2(j0, j - j0);
+      ++n;
+      j0 = j;
+    }
+  if (count) count[b] = n;
 }
 
 }  // namespace
@@ -790,6 +816,9 @@ LsqrDev Lsqr::view() const {
   d.cp = cp_.as<int>();
   d.crow = crow_.as<int>();
   d.cval = cval_.as<double>();
+  d.task = task_.as<int2>();
+  d.ntask = ntask_;
+  d.task_log = task_log_;
   d.nb = nb_.as<int4>();
   d.if_start = if_start_;
   d.if_n = if_n_;
@@ -871,6 +900,33 @@ std::string Lsqr::build_csc() {
   if (nvalid > 0)
     k_csc_fill<<<grid_, kLsThreads, 0, st_>>>(perm.as<int>(), row_of.as<int>(), val_.as<double>(),
                                               nvalid, crow_.as<int>(), cval_.as<double>());
+  LCK(cudaGetLastError());
+  return build_tasks();
+}
+
+std::string Lsqr::build_tasks() {
+  task_log_ = rows_log(np_, grid_ * (kLsThreads / 32));
+  const int nblock = (np_ + (1 << task_log_) - 1) >> task_log_;
+  DevBuf cnt, first, tmp;
+  cnt.alloc((size_t)(nblock + 1) * 4);
+  first.alloc((size_t)(nblock + 1) * 4);
+  if (!cnt.p || !first.p) return "device allocation failed (column runs)";
+  LCK(cudaMemsetAsync(cnt.p, 0, (size_t)(nblock + 1) * 4, st_));
+  const int blocks = (nblock + 127) / 128;
+  k_tasks<<<blocks, 128, 0, st_>>>(cp_.as<int>(), np_, task_log_, nblock, cnt.as<int>(), nullptr,
+                                   nullptr);
+  size_t bytes = 0;
+  LCK(cub::DeviceScan::ExclusiveSum(nullptr, bytes, cnt.as<int>(), first.as<int>(), nblock + 1,
+                                    st_));
+  tmp.alloc(std::max<size_t>(bytes, 16));
+  if (!tmp.p) return "device allocation failed (column runs)";
+  LCK(cub::DeviceScan::ExclusiveSum(tmp.p, bytes, cnt.as<int>(), first.as<int>(), nblock + 1, st_));
+  LCK(cudaMemcpyAsync(&ntask_, first.as<int>() + nblock, 4, cudaMemcpyDeviceToHost, st_));
+  LCK(cudaStreamSynchronize(st_));
+  task_.alloc((size_t)std::max(ntask_, 1) * sizeof(int2));
+  if (!task_.p) return "device allocation failed (column runs)";
+  k_tasks<<<blocks, 128, 0, st_>>>(cp_.as<int>(), np_, task_log_, nblock, nullptr, first.as<int>(),
+                                   task_.as<int2>());
   LCK(cudaGetLastError());
   LCK(cudaStreamSynchronize(st_));
   return std::string();

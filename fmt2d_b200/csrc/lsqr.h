@@ -66,6 +66,9 @@ struct LsqrDev {
   // smooth_type and, for 2 and 3, the Gaussian operators: R_h, R_v and their
   // transposes, the interface R_h (applied as its own adjoint, as the
   // reference does)
+  // the columns in runs for a warp each (build_tasks): first column and number
+  const int2* task = nullptr;
+  int ntask = 0, task_log = 0;
   int stype = 1;
   SpRows rh, rht, rv, rvt, ri;
   const double* residual = nullptr;
@@ -137,6 +140,9 @@ class Lsqr {
   int nd_ = 0, np_ = 0, nvp_ = 0, if_start_ = 0, if_n_ = 0;
   long long nnz_ = 0;
   int grid_ = 0, grid3_ = 0;   // blocks (smooth_type 1 and 2; 3)
+  DevBuf task_;                // LsqrDev::task
+  int ntask_ = 0, task_log_ = 0;
+  std::string build_tasks();
   DevBuf rp_, col_, val_, cp_, crow_, cval_, nb_, mask_, res_, dms_, gtg_, u_, v_, w_, dm_,
       part_, sc_, x_, y_;
   // smoothing matrices: R_h, R_h^T, R_v, R_v^T, interface R_h
