@@ -735,36 +735,66 @@ __device__ __forceinline__ void list_start(const Fld64& F, unsigned s) {
 }
 
 // Fixed-point check of every node (window ignored): a node whose update
-// would change it is listed and counted.  Nodes at an interface are evaluated
-// by evaluate(), on the state as it was unpacked; the regular ones, which are
-// nearly all and cost a dozen roots and quotients there, by reg_best on the
-// records the state came from (60 fields of 800,000 nodes: 4.8 -> 3.0 ms).
-__global__ void k_verify(Fld64* fields, int nf) {
+// would change it is listed and counted.  The regular nodes, which are nearly
+// all and cost evaluate() a dozen roots and quotients each, are evaluated by
+// reg_best on the records the state came from.
+__device__ __forceinline__ bool regular_slot(const Fld64& F, int s) {
+  constexpr uint32_t kPlain = kInRegion | kUpdatable | kFullyRegular;
+  return (F.code[s] & kPlain) == kPlain && s < F.H * F.pitch;
+}
+
+__global__ void __launch_bounds__(256) k_verify(Fld64* fields, int nf) {
   const Fld64& F = fields[blockIdx.y];
   const int ns = F.nslots();
   const double rdx = 1.0 / F.dx;
-  constexpr uint32_t kPlain = kInRegion | kUpdatable | kFullyRegular;
   unsigned nbad = 0;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < ns; s += gridDim.x * blockDim.x) {
     const int row = s / F.pitch, col = s - row * F.pitch;
-    if (col >= F.nx) continue;
-    NewV nv;
-    if ((F.code[s] & kPlain) == kPlain && row < F.H) {
-      if (s == F.frozen_slot) continue;
-      const Rec me = load_rec(F, s);
-      Self self;
-      self.T = me.T;
-      self.g = make_double2(me.gx, me.gz);
-      self.fl = F.fl[s];
-      const RegBest rb = reg_best<false>(F, rdx, s, row, col, fabs(me.v), 15u);
-      nv = settle(F, s, rb.t, rb.gx, rb.gz, false, rb.key != kNoKey && !(rb.key & 1), rb.t, self);
-    } else {
-      nv = evaluate(F, s);
-    }
+    if (col >= F.nx || !regular_slot(F, s) || s == F.frozen_slot) continue;
+    const Rec me = load_rec(F, s);
+    Self self;
+    self.T = me.T;
+    self.g = make_double2(me.gx, me.gz);
+    self.fl = F.fl[s];
+    const RegBest rb = reg_best<false>(F, rdx, s, row, col, fabs(me.v), 15u);
+    const NewV nv =
+        settle(F, s, rb.t, rb.gx, rb.gz, false, rb.key != kNoKey && !(rb.key & 1), rb.t, self);
     if (nv.write) {
       ++nbad;
       list_start(F, (unsigned)s);
     }
+  }
+  if (nbad) atomicAdd(F.cnt + 1, nbad);
+}
+
+// The nodes at an interface, by evaluate() on the state as it was unpacked.
+// A block gathers those of its slots first: one is a chain of 57,000 cycles, and
+// left where they are each holds a warp of others.  (60 fields of 800,000 nodes:
+// both kernels 1.9 ms, one kernel for all nodes 3.0, evaluate() alone 4.8.  A
+// longer span gathers better, 1.7 ms at 4096, but leaves a small field's nodes to a
+// few blocks: 121 x 66 nodes, five fields, 7% slower.)
+constexpr int kCheckSpan = 512;
+__global__ void __launch_bounds__(128) k_verify_cut(Fld64* fields, int nf) {
+  const Fld64& F = fields[blockIdx.y];
+  const int ns = F.nslots();
+  __shared__ unsigned list[kCheckSpan];
+  __shared__ unsigned n;
+  unsigned nbad = 0;
+  for (int b = blockIdx.x * kCheckSpan; b < ns; b += gridDim.x * kCheckSpan) {
+    if (threadIdx.x == 0) n = 0;
+    __syncthreads();
+    for (int s = b + threadIdx.x; s < min(b + kCheckSpan, ns); s += blockDim.x)
+      if ((s % F.pitch) < F.nx && (F.code[s] & kInRegion) && !regular_slot(F, s))
+        list[atomicAdd(&n, 1u)] = (unsigned)s;
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
+      const NewV nv = evaluate(F, (int)list[i]);
+      if (nv.write) {
+        ++nbad;
+        list_start(F, list[i]);
+      }
+    }
+    __syncthreads();
   }
   if (nbad) atomicAdd(F.cnt + 1, nbad);
 }
@@ -1195,6 +1225,8 @@ void e64_solve(Fld64* f, const Fld64* fh, int nf, size_t max_slots, bool windowe
 void e64_verify(Fld64* f, int nf, size_t max_slots, cudaStream_t st) {
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 512);
   k_verify<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
+  const int bc = (int)std::min<size_t>((max_slots + kCheckSpan - 1) / kCheckSpan, 2048);
+  k_verify_cut<<<dim3(bc, nf), 128, 0, st>>>(f, nf);
 }
 void e64_finish(Fld64* f, int nf, size_t max_slots, const int* water_up, cudaStream_t st) {
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 512);
