@@ -457,7 +457,12 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
       if (live && !in_sh) cov[j - kCCap] = lose ? s | kCutBit : e & ~kCutBit;
     }
     __syncthreads();
-    if (tid == 0) lap(1);
+    if (tid == 0) {
+      // (all have read it before this barrier; the next commits come after the
+      // one that ends the step)
+      sh.nc = 0;
+      lap(1);
+    }
     // spread: every candidate of a node u that involves node v is at or above
     // v's time, so a change of v from a to b can only move nodes at or above
     // min(a, b); those below are not listed unless they wait with a time
@@ -620,7 +625,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
     }
     __syncthreads();
     if (tid == 0) {
-      sh.nc = sh.nw[0] = sh.nw[1] = 0u;
+      sh.nw[0] = sh.nw[1] = 0u;
       lap(3);
     }
     // the window moves on after a step that changed nothing inside it (or
