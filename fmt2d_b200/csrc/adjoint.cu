@@ -1281,12 +1281,8 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
   constexpr size_t kPerSlot = sizeof(AdjLink) + sizeof(AdjNode) + 2 * sizeof(unsigned) + 3 * sizeof(double) +
                               2 * sizeof(unsigned) + 2 * sizeof(unsigned) +
                               4 * sizeof(AdjRead);
-  size_t free_b = 0, total_b = 0;
-  ACK(cudaMemGetInfo(&free_b, &total_b));
-  const size_t budget = (free_b + adjspace_.bytes()) / 2;
-  // (the chunk's state stays: 15 GB for 90 fields of 800,000 nodes, which took
-  // 25 ms a call to allocate and free)
-  const Spare::Use use(adjspace_, 8);
+  const CallMem mem(pool_.get(), stream_);
+  const size_t budget = mem.avail / 2;
   unsigned long long cnt_bad = 0, cnt_unl = 0, cnt_left = 0, cnt_reach = 0, cnt_fields = 0;
   unsigned max_rounds = 0;
   int s0 = 0;
@@ -1320,9 +1316,8 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
     for (int i = 0; i < nf; ++i) off[i + 1] = off[i] + reg_[kTf[items[i].tf].reg].nslots;
     const size_t tot = off[nf];
     DevBuf b_ctr, b_gz;
-    AdjSpace& W = adjspace_;
-    DevBuf &b_link = W.link, &b_node = W.node, &b_cnt = W.cnt, &b_lam = W.lam, &b_d = W.d,
-           &b_gv = W.gv, &b_fa = W.fa, &b_fb = W.fb, &b_rcnt = W.rcnt, &b_roff = W.roff;
+    CallBuf b_link(mem), b_node(mem), b_cnt(mem), b_lam(mem), b_d(mem), b_gv(mem), b_fa(mem),
+        b_fb(mem), b_rcnt(mem), b_roff(mem), b_rd(mem);
     b_rcnt.alloc(tot * sizeof(unsigned));
     b_roff.alloc(tot * sizeof(unsigned));
     b_gz.alloc((size_t)nf * 3 * m_.nx * sizeof(double));
@@ -1507,7 +1502,6 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
                           stream_));
       ACK(cudaStreamSynchronize(stream_));
       const size_t nref = (size_t)last[0] + last[1];
-      DevBuf& b_rd = W.rd;
       b_rd.alloc(std::max<size_t>(nref, 1) * sizeof(AdjRead));
       if (!b_rd.p) return "device allocation failed (reader lists)";
       adj_readers(dA + i0, i1 - i0, max_slots, b_rd.as<AdjRead>(), stream_);

@@ -44,12 +44,10 @@ unsigned phase_fields(int mask) {
 void DevBuf::alloc(size_t n) {
   if (n <= bytes && p) return;
   free_();
-  for (int tries = 0;; ++tries) {
-    if (cudaMalloc(&p, n < 16 ? 16 : n) == cudaSuccess) break;
+  if (cudaMalloc(&p, n < 16 ? 16 : n) != cudaSuccess) {
     cudaGetLastError();   // the caller's to report: not the next launch check's
     p = nullptr;
-    bytes = 0;
-    if (tries || !Spare::reclaim()) return;
+    return;
   }
   bytes = n;
 }
@@ -60,50 +58,80 @@ void DevBuf::free_() {
   bytes = 0;
 }
 
-namespace {
-std::mutex g_spare_mu;
-std::vector<Spare*>& spares() {
-  static std::vector<Spare*>* v = new std::vector<Spare*>;   // (outlives every engine)
-  return *v;
-}
-}  // namespace
-
-void Spare::leave() {
-  std::lock_guard<std::mutex> lock(g_spare_mu);
-  auto& v = spares();
-  const auto it = std::find(v.begin(), v.end(), this);
-  if (it != v.end()) v.erase(it);
-}
-size_t Spare::bytes() const {
-  size_t n = 0;
-  for (const DevBuf* b : bufs_) n += b->bytes;
-  return n;
-}
-void Spare::release() {
-  for (DevBuf* b : bufs_) b->free_();
-}
-bool Spare::reclaim() {
-  std::lock_guard<std::mutex> lock(g_spare_mu);
-  bool any = false;
-  for (Spare* s : spares())
-    if (!s->busy_ && s->bytes() > 0) {
-      s->release();
-      any = true;
-    }
-  return any;
-}
-Spare::Use::Use(Spare& s, int share) : s_(s), share_(share) {
-  std::lock_guard<std::mutex> lock(g_spare_mu);
-  s_.busy_ = true;
-  auto& v = spares();
-  if (std::find(v.begin(), v.end(), &s_) == v.end()) v.push_back(&s_);
-}
-Spare::Use::~Use() {
+std::shared_ptr<WorkPool> WorkPool::of(int device) {
+  static std::mutex mu;
+  static std::weak_ptr<WorkPool> pools[64];
+  if (device < 0 || device >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (std::shared_ptr<WorkPool> p = pools[device].lock()) return p;
+  int can = 0;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) total_b = 0;
-  std::lock_guard<std::mutex> lock(g_spare_mu);
-  if (s_.bytes() > total_b / share_) s_.release();
-  s_.busy_ = false;
+  cudaDeviceGetAttribute(&can, cudaDevAttrMemoryPoolsSupported, device);
+  if (!can || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  props.maxSize = total_b / kShare;
+  std::shared_ptr<WorkPool> p(new WorkPool);
+  unsigned long long keep = ~0ull;   // (all of it: the pool itself is bounded)
+  if (cudaMemPoolCreate(&p->pool_, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(p->pool_, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  pools[device] = p;
+  return p;
+}
+
+WorkPool::~WorkPool() {
+  if (pool_) cudaMemPoolDestroy(pool_);
+}
+
+size_t WorkPool::idle() const {
+  unsigned long long held = 0, used = 0;
+  if (cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return held > used ? (size_t)(held - used) : 0;
+}
+
+CallMem::CallMem(const WorkPool* p, cudaStream_t stream) : st(stream) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  avail = free_b + (p ? p->idle() : 0);
+  if (p && avail >= total_b / 4) pool = p->handle();
+}
+
+void CallBuf::alloc(size_t n) {
+  if (n <= bytes && p) return;
+  free_();
+  if (n < 16) n = 16;
+  pooled_ = m_->pool && cudaMallocFromPoolAsync(&p, n, m_->pool, m_->st) == cudaSuccess;
+  if (!pooled_) {
+    cudaGetLastError();   // (also of the pool's attempt)
+    if (cudaMalloc(&p, n) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return;
+    }
+  }
+  bytes = n;
+}
+
+void CallBuf::free_() {
+  if (p && pooled_) cudaFreeAsync(p, m_->st);
+  else if (p) cudaFree(p);
+  p = nullptr;
+  bytes = 0;
 }
 
 namespace {
@@ -176,6 +204,7 @@ double seafloor_at(const Model& m, double px) {
 
 Engine::Engine(int device) : device_(device) {
   cudaSetDevice(device_);
+  pool_ = WorkPool::of(device_);
   cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
   cudaEventCreateWithFlags(&ev_start_, cudaEventDisableTiming);
   for (SolveLane& L : lanes_) {

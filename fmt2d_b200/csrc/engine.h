@@ -48,33 +48,58 @@ struct DevBuf {
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
 
-// Buffers an engine keeps from one call for the next.  When a call is over
-// (Use's end) they stay only if they take no more than a share of the device's
-// memory, and while no call uses them any allocation of the library that finds
-// no memory takes them back (reclaim, from any engine and thread).
-class Spare {
+// The driver's memory pool that calls take their large workspaces from, one
+// per device, shared by its engines and gone with the last of them.  What no
+// call uses stays in it, at most a share of the device, for the next call of
+// any engine, and the driver gives it to whatever allocation of the process
+// (PyTorch's too) finds no memory otherwise.  (A gradient of 90 fields of
+// 800,000 nodes works in 15 GB: 25 to 60 ms to allocate and free, 0.03 ms from
+// the pool; the pool's own growth is 6 ms a GB, once.)
+class WorkPool {
  public:
-  Spare() = default;
-  Spare(const Spare&) = delete;
-  Spare& operator=(const Spare&) = delete;
-  size_t bytes() const;
-  class Use {
-   public:
-    Use(Spare& s, int share);
-    ~Use();
-   private:
-    Spare& s_;
-    int share_;
-  };
-  static bool reclaim();   // whether anything was freed
-
- protected:
-  std::vector<DevBuf*> bufs_;
-  void leave();            // before the buffers go
+  static constexpr size_t kShare = 8;                // of the device's memory: one eighth
+  static std::shared_ptr<WorkPool> of(int device);   // null: no pools on this device
+  ~WorkPool();
+  WorkPool(const WorkPool&) = delete;
+  WorkPool& operator=(const WorkPool&) = delete;
+  cudaMemPool_t handle() const { return pool_; }
+  size_t idle() const;                               // bytes held that no call uses
 
  private:
-  void release();
-  bool busy_ = false;
+  WorkPool() = default;
+  cudaMemPool_t pool_ = nullptr;
+};
+
+// A call's view of the device's memory: what it can have, and whether its
+// buffers come from the pool.  Where less than a quarter of the device is to be
+// had, they are allocated and freed one by one (exactly what is needed, and
+// nothing stays).
+struct CallMem {
+  CallMem() = default;
+  CallMem(const WorkPool* pool, cudaStream_t st);
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t st = nullptr;
+  size_t avail = 0;
+};
+
+// A buffer of one call, used on the call's stream and freed in its order.
+// (Beyond the pool's bound, and where the pool finds no memory, an allocation
+// of its own.)
+class CallBuf {
+ public:
+  explicit CallBuf(const CallMem& m) : m_(&m) {}
+  ~CallBuf() { free_(); }
+  CallBuf(const CallBuf&) = delete;
+  CallBuf& operator=(const CallBuf&) = delete;
+  void alloc(size_t n);
+  template <class T> T* as() const { return static_cast<T*>(p); }
+  void* p = nullptr;
+  size_t bytes = 0;
+
+ private:
+  void free_();
+  const CallMem* m_;
+  bool pooled_ = false;
 };
 
 // Static device data of one region (slot layout of model.h).
@@ -205,6 +230,7 @@ class Engine {
   Fld64 field_view(int src, int tf) const;
   int device_;
   cudaStream_t stream_ = nullptr;
+  std::shared_ptr<WorkPool> pool_;
   Model m_;
   DevRegionStore reg_[7];
   DevBuf ifc_buf_[6][6];      // z, nx, nz, vel_top, vel_bot, izc
@@ -225,19 +251,6 @@ class Engine {
   DevBuf d_pvel_, d_invidx_, d_xpos_, d_picks_, d_trfields_, d_srcx_, d_srcz_,
       d_tcalc_, d_valid_, d_cnt_, d_off_, d_rowptr_, d_tmp_, d_col_, d_val_, d_sft_, d_sfjobs_,
       d_entry_;
-  // Frechet rows' workspace: sort keys and values, the pool of the rays'
-  // entries (the sort's second buffers later), its chunks' owners and counter
-  struct RowSpace : Spare {
-    DevBuf keys, vals, ids, pvals, owner, used;
-    RowSpace() { bufs_ = {&keys, &vals, &ids, &pvals, &owner, &used}; }
-    ~RowSpace() { leave(); }
-  } rowspace_;
-  // The adjoint's state of a chunk of sources (misfit_gradient)
-  struct AdjSpace : Spare {
-    DevBuf link, node, cnt, lam, d, gv, fa, fb, rcnt, roff, rd;
-    AdjSpace() { bufs_ = {&link, &node, &cnt, &lam, &d, &gv, &fa, &fb, &rcnt, &roff, &rd}; }
-    ~AdjSpace() { leave(); }
-  } adjspace_;
   int npick_ = -1, rows_ = 0;
   long long nnz_ = 0;
   double trace_ms_ = 0.0;

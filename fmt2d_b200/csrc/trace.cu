@@ -190,8 +190,13 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
     // the pool: entries of a ray as long as its offset and the model's depth
     // twice (four a cell); where that is too little, or memory is short, the
     // rays that count their entries are traced again into one of the right size
-    RowSpace& W = rowspace_;
-    const Spare::Use use(W, 16);
+    // (sort keys and values; the rays' entries, which the sort's second buffers
+    // take the place of, their chunks' owners and counter)
+    const CallMem mem = rows ? CallMem(pool_.get(), stream_) : CallMem();
+    struct RowSpace {
+      CallBuf keys, vals, ids, pvals, owner, used;
+      explicit RowSpace(const CallMem& m) : keys(m), vals(m), ids(m), pvals(m), owner(m), used(m) {}
+    } W(mem);
     size_t chunks = 0;
     TrPool pool;
     auto set_pool = [&](size_t n) {
@@ -216,10 +221,7 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
       chunks = (size_t)(4.0 * len / kTrChunk) + (size_t)npick;
       W.used.alloc(sizeof(unsigned));
       if (!W.used.p) return "device allocation failed (Frechet)";
-      size_t free_b = 0, total_b = 0;
-      TCK(cudaMemGetInfo(&free_b, &total_b));
-      const size_t fit = (free_b / 4 + W.ids.bytes + W.pvals.bytes + W.owner.bytes) /
-                         (kTrChunk * 16 + sizeof(uint2));
+      const size_t fit = mem.avail / 4 / (kTrChunk * 16 + sizeof(uint2));
       // (no memory for a pool: the rays are counted)
       set_pool(std::min({chunks, fit, (size_t)(0x7fffffffu / kTrChunk) + npick}));
       pool.used = W.used.as<unsigned>();

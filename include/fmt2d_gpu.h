@@ -32,6 +32,13 @@
  * (1 Pg, 2 PsedP, 3 PmP, 4 Pg_ss, 5 Pg_ss2) and time-field ids (1..12) follow
  * the reference's numbering.  One context per host thread; calls on a context
  * are ordered on its CUDA stream.  All arrays are caller-owned host memory.
+ *
+ * Device memory: a context holds its model and the fields of its last forward.
+ * fmt2d_trace and fmt2d_misfit_gradient take their workspaces from a driver
+ * memory pool that the contexts of a device share.  It holds on to at most an
+ * eighth of the device's memory between calls; the driver hands what no call
+ * uses to any allocation of the process that would otherwise fail, and the pool
+ * goes with the device's last context.
  */
 #ifndef FMT2D_GPU_H
 #define FMT2D_GPU_H
