@@ -120,6 +120,7 @@ def lib():
     L.fmt2d_forward_batch.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p,
                                       C.c_void_p]
     L.fmt2d_set_solve_threads.argtypes = [V, C.c_int]
+    L.fmt2d_set_full_check.argtypes = [V, C.c_int]
     L.fmt2d_set_param_grid.argtypes = [V, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_int]
     L.fmt2d_trace_entries.argtypes = [V, C.c_void_p, C.c_void_p, C.c_void_p]
     L.fmt2d_misfit_gradient.argtypes = [V, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,

@@ -501,6 +501,12 @@ class Fmt2d:
                                               int(max_steps)), "fmt2d_set_schedule")
         return self
 
+    def set_full_check(self, on: bool = True):
+        """Check every node of a solved field with the one-thread stencil, which
+        shares nothing with the solver's evaluation (fmt2d_set_full_check)."""
+        self._check(self.L.fmt2d_set_full_check(self.h, int(bool(on))), "fmt2d_set_full_check")
+        return self
+
     def set_solve_threads(self, threads: int = 0):
         """Threads of each field's solve block (fmt2d_set_solve_threads): 256,
         384 or 512, 0 for the default; results are identical for every size."""

@@ -565,6 +565,14 @@ int fmt2d_set_iface_window(fmt2d_ctx* ctx, double cells) {
   return FMT2D_OK;
 }
 
+int fmt2d_set_full_check(fmt2d_ctx* ctx, int on) {
+  if (!ctx) return FMT2D_ERR_ARG;
+  int code = 0;
+  if (!ctx->need_gpu(code)) return code;
+  ctx->eng->check_all = on != 0;
+  return FMT2D_OK;
+}
+
 int fmt2d_set_solve_threads(fmt2d_ctx* ctx, int threads) {
   if (!ctx) return FMT2D_ERR_ARG;
   int code = 0;

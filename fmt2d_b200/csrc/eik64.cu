@@ -742,7 +742,9 @@ __device__ __forceinline__ void list_start(const Fld64& F, unsigned s) {
 // Fixed-point check of every node (window ignored): a node whose update
 // would change it is listed and counted.  The regular nodes, which are nearly
 // all and cost evaluate() a dozen roots and quotients each, are evaluated by
-// reg_best on the records the state came from.
+// reg_best on the records the state came from: the solver's own function, so
+// this finds nodes that were not evaluated again, not an error of reg_best.
+// k_verify_cut<true> evaluates every node with evaluate() instead.
 __device__ __forceinline__ bool regular_slot(const Fld64& F, int s) {
   constexpr uint32_t kPlain = kInRegion | kUpdatable | kFullyRegular;
   return (F.code[s] & kPlain) == kPlain && s < F.H * F.pitch;
@@ -772,13 +774,15 @@ __global__ void __launch_bounds__(256) k_verify(Fld64* fields, int nf) {
   if (nbad) atomicAdd(F.cnt + 1, nbad);
 }
 
-// The nodes at an interface, by evaluate() on the state as it was unpacked.
+// The nodes at an interface (kAll: every node), by evaluate() on the state as it
+// was unpacked.
 // A block gathers those of its slots first: one is a chain of 57,000 cycles, and
 // left where they are each holds a warp of others.  (60 fields of 800,000 nodes:
 // both kernels 1.9 ms, one kernel for all nodes 3.0, evaluate() alone 4.8.  A
 // longer span gathers better, 1.7 ms at 4096, but leaves a small field's nodes to a
 // few blocks: 121 x 66 nodes, five fields, 7% slower.)
 constexpr int kCheckSpan = 512;
+template <bool kAll>
 __global__ void __launch_bounds__(128) k_verify_cut(Fld64* fields, int nf) {
   const Fld64& F = fields[blockIdx.y];
   const int ns = F.nslots();
@@ -789,7 +793,8 @@ __global__ void __launch_bounds__(128) k_verify_cut(Fld64* fields, int nf) {
     if (threadIdx.x == 0) n = 0;
     __syncthreads();
     for (int s = b + threadIdx.x; s < min(b + kCheckSpan, ns); s += blockDim.x)
-      if ((s % F.pitch) < F.nx && (F.code[s] & kInRegion) && !regular_slot(F, s))
+      if ((s % F.pitch) < F.nx && (F.code[s] & kInRegion) &&
+          (kAll || !regular_slot(F, s)))
         list[atomicAdd(&n, 1u)] = (unsigned)s;
     __syncthreads();
     for (unsigned i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1227,11 +1232,15 @@ void e64_solve(Fld64* f, const Fld64* fh, int nf, size_t max_slots, bool windowe
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 1024);
   k_unpack<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
 }
-void e64_verify(Fld64* f, int nf, size_t max_slots, cudaStream_t st) {
+void e64_verify(Fld64* f, int nf, size_t max_slots, bool all, cudaStream_t st) {
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 512);
-  k_verify<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
   const int bc = (int)std::min<size_t>((max_slots + kCheckSpan - 1) / kCheckSpan, 2048);
-  k_verify_cut<<<dim3(bc, nf), 128, 0, st>>>(f, nf);
+  if (all) {
+    k_verify_cut<true><<<dim3(bc, nf), 128, 0, st>>>(f, nf);
+    return;
+  }
+  k_verify<<<dim3(bx, nf), 256, 0, st>>>(f, nf);
+  k_verify_cut<false><<<dim3(bc, nf), 128, 0, st>>>(f, nf);
 }
 void e64_finish(Fld64* f, int nf, size_t max_slots, const int* water_up, cudaStream_t st) {
   const int bx = (int)std::min<size_t>((max_slots + 255) / 256, 512);

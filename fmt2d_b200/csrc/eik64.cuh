@@ -109,8 +109,8 @@ const int* e64_solve_sizes(int* n);
 int e64_tiles(const Fld64& f);
 int e64_tiles_max();
 // Fixed-point check of every node: a node whose evaluation would change it
-// is listed in list_in and counted in cnt[1].
-void e64_verify(Fld64* f, int nf, size_t max_slots, cudaStream_t st);
+// is listed in list_in and counted in cnt[1].  all: by the one-thread stencil.
+void e64_verify(Fld64* f, int nf, size_t max_slots, bool all, cudaStream_t st);
 void e64_finish(Fld64* f, int nf, size_t max_slots, const int* water_up, cudaStream_t st);
 // PmP head-wave sweep of the selected fields; pre (device array of nsel
 // pointers, may be null, entries may be null) receives each field's solved

@@ -583,8 +583,8 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
     L.stats.launches += 2;
     ++L.stats.final_passes;
     cudaMemsetAsync(L.sinq.p, 0, words * sizeof(unsigned), L.st);
-    e64_verify(dF, nf, max_slots, L.st);
-    L.stats.launches += 2;
+    e64_verify(dF, nf, max_slots, check_all, L.st);
+    L.stats.launches += check_all ? 1 : 2;
     cudaError_t ce = cudaMemcpyAsync(hc, L.scnt.p, (size_t)nf * 4 * sizeof(unsigned),
                                      cudaMemcpyDeviceToHost, L.st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(L.st);

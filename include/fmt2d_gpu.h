@@ -407,6 +407,13 @@ FMT2D_API int fmt2d_set_schedule(fmt2d_ctx* ctx, double window_cells, int max_pa
  * of solver steps does. */
 FMT2D_API int fmt2d_set_iface_window(fmt2d_ctx* ctx, double cells);
 
+/* How a forward checks its fields (after every solve pass, every node).  0, the
+ * default: regular nodes are evaluated as the solver does, those at an
+ * interface by the one-thread stencil.  Otherwise every node by the one-thread
+ * stencil, which forms all its candidates: independent of the solver, and slower
+ * (a diagnostic).  No reference counterpart. */
+FMT2D_API int fmt2d_set_full_check(fmt2d_ctx* ctx, int on);
+
 /* Threads of each field's solve block: 256, 384 or 512 (0: the default,
  * 384).  Results are the same bit for bit for every size (no evaluation of a
  * solve step sees a value written in that step); only the time differs: larger
