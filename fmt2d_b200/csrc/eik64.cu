@@ -89,6 +89,7 @@ struct SolvePlan {
   int tiles;       // tiles of the largest field if a field has a window, else 0
   int mwords;      // moving bitmap: words per row (a power of two), and in all
   int mtotal;
+  unsigned rmask;  // its rows: slot row & rmask
 };
 
 // Solve every field of the batch from its list_in (one block per field).
@@ -97,10 +98,10 @@ struct SolvePlan {
 // thread evaluates one of the former or the regular quadrants of one of the
 // latter, then sixteen lanes evaluate a node's cut cells (eik_coop.cuh).
 //
-// The nodes that move in a step mark a small bitmap (all rows, columns modulo
-// 32 * mwords) and claim their new time in global memory with the step's
-// stamp; a node looks up only the claims of marked neighbours, and the stamp
-// tells a mark of another column or step.
+// The nodes that move in a step mark a small bitmap (rows modulo rmask + 1,
+// columns modulo 32 * mwords) and claim their new time in global memory with the
+// step's stamp; a node looks up only the claims of marked neighbours, and the
+// stamp tells a mark of another row, column or step.
 //
 // Waiting nodes: a node whose new time lies beyond the window records it in
 // pend and sets its bit in the waiting bitset; each tile of 8 x 32 slots
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
         sh.changed[par] = 1;
         F.claim[s] = make_ulonglong2(dbits(nv.T), stamp);
         const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
-        atomicOr(mbits + (unsigned)row * P.mwords + ((col >> 5) & mmask), 1u << (col & 31));
+        atomicOr(mbits + ((unsigned)row & P.rmask) * P.mwords + ((col >> 5) & mmask), 1u << (col & 31));
       }
     };
     const unsigned nr = sh.cnt[cur][0], nx = sh.cnt[cur][1];
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
         // marks of columns c0 .. c0 + 4 of a slot row
         auto marks = [&](int r, unsigned which) -> unsigned long long {
           if (r < 0 || r >= F.H + 2) return 0ull;
-          const unsigned* m = mbits + (unsigned)r * P.mwords;
+          const unsigned* m = mbits + ((unsigned)r & P.rmask) * P.mwords;
           const int c0 = col - 2, w = c0 >> 5;
           return __funnelshift_r(m[w & mmask], m[(w + 1) & mmask], c0 & 31) & which;
         };
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
       const unsigned e = j < kCCap ? ce[j] : cov[j - kCCap];
       const unsigned s = e & kSlotMask;
       const int row = row_of(s), col = (int)(s - (unsigned)row * pitch);
-      mbits[(unsigned)row * P.mwords + ((col >> 5) & mmask)] = 0u;
+      mbits[((unsigned)row & P.rmask) * P.mwords + ((col >> 5) & mmask)] = 0u;
     }
     __syncthreads();
     if (tid == 0) {
@@ -1203,6 +1204,7 @@ static void solve_launch(Fld64* f, const Fld64* fh, int nf, bool windowed, long 
   // eight (256 columns: marks of other columns are then rare)
   const size_t room = solve_room<NT>();
   P.nbits = windowed ? 2 : 1;
+  P.rmask = ~0u;
   for (;; --P.nbits) {
     for (P.mwords = 8; P.mwords > 1; P.mwords /= 2) {
       P.mtotal = rows * P.mwords;
@@ -1210,6 +1212,12 @@ static void solve_launch(Fld64* f, const Fld64* fh, int nf, bool windowed, long 
     }
     P.mtotal = rows * P.mwords;
     if (P.nbits == 0 || solve_smem(P) <= room) break;
+  }
+  // more rows than words of shared memory (regions of tens of thousands of rows,
+  // which only a narrow model has): rows that lie 2^k apart share a word
+  for (unsigned r = 1u << 30; solve_smem(P) > room && r >= 64u; r >>= 1) {
+    P.rmask = r - 1;
+    P.mtotal = std::min(rows, (int)r);
   }
   k_solve<NT><<<nf, NT, solve_smem(P), st>>>(f, P, max_steps, ctr);
 }

@@ -585,8 +585,10 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
     cudaMemsetAsync(L.sinq.p, 0, words * sizeof(unsigned), L.st);
     e64_verify(dF, nf, max_slots, check_all, L.st);
     L.stats.launches += check_all ? 1 : 2;
-    cudaError_t ce = cudaMemcpyAsync(hc, L.scnt.p, (size_t)nf * 4 * sizeof(unsigned),
-                                     cudaMemcpyDeviceToHost, L.st);
+    cudaError_t ce = cudaGetLastError();
+    if (ce == cudaSuccess)
+      ce = cudaMemcpyAsync(hc, L.scnt.p, (size_t)nf * 4 * sizeof(unsigned), cudaMemcpyDeviceToHost,
+                           L.st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(L.st);
     if (ce != cudaSuccess) { err = std::string("eikonal solve: ") + cudaGetErrorString(ce); break; }
     bad = 0;
