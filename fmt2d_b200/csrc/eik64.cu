@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1)
   const unsigned mmask = (unsigned)P.mwords - 1u;
   // lists: regular nodes overflow to the front of the list's part of over,
   // the others to its back (together at most the field's slots)
-  unsigned* cov = F.over + 2 * (size_t)ns;
+  // (the start list has been read when the first commit is made)
+  unsigned* cov = F.list_in;
   // a field without a window never holds a node back: nothing waits
   const bool windowed = F.clock[1] < kReachD;
   // The collective steps below are called by whole warps: places in a list or
@@ -855,11 +856,10 @@ __global__ void k_fill(Fld64* fields, int nf) {
        i += (size_t)gridDim.x * blockDim.x) {
     F.T[i] = kHugeD;
     F.G[i] = make_double2(0.0, 0.0);
-    F.Gout[i] = make_double2(0.0, 0.0);
+    F.claim[i] = make_ulonglong2(0, 0);   // of no step (the bits of Gout's zeros)
     F.seed[i] = make_double4(kHugeD, 0.0, 0.0, 0.0);
     F.fl[i] = 0;
     F.pend[i] = -1.0;
-    F.claim[i] = make_ulonglong2(0, 0);   // of no step
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     F.frozen_slot = -1;

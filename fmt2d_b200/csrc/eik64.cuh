@@ -41,8 +41,10 @@ struct Fld64 {
   uint8_t* fln = nullptr;
   double* pend = nullptr;           // time a deferred node waits with (< 0: none)
   ulonglong2* claim = nullptr;      // of a node that moves: bits of its new time, the step
-  unsigned* list_in = nullptr;      // nodes to start from (seeds, re-listed nodes)
-  unsigned* over = nullptr;         // 3*nslots: overflow of the two lists and of the commits
+                                    // (in Gout's place until the solve is over)
+  unsigned* list_in = nullptr;      // nodes to start from (seeds, re-listed nodes); during
+                                    // the steps overflow of the commits
+  unsigned* over = nullptr;         // 2*nslots: overflow of the two lists
   unsigned* inq = nullptr;          // bitset over slots: listed (when not in shared memory)
   unsigned* wait = nullptr;         // bitset over slots: waiting (when not in shared memory)
   unsigned* cnt = nullptr;          // [0] list_in length, [1] unsettled nodes found by a check,

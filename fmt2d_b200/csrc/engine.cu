@@ -466,21 +466,18 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
     std::string e0s = lane_reserve(L, (size_t)nf * per + kCtrN * 8 + 16 * 256);
     if (!e0s.empty()) return e0s;
   }
-  // solver scratch of the batch, per slot: staged time, gradient and flags,
-  // pending time, start list, list and commit overflow, listed bitset
+  // solver scratch of the batch, per slot: record, staged flags, pending time,
+  // start list and commit overflow, overflow of the two lists, two bitsets
   const size_t words = (total + 31 * (size_t)nf + 31) / 32 + (size_t)nf;
   L.sR.alloc(total * sizeof(double4));
   L.sfln.alloc(total);
   L.spend.alloc(total * sizeof(double));
-  L.sclaim.alloc(total * sizeof(ulonglong2));
   L.slist.alloc(total * sizeof(unsigned));
-  L.sover.alloc(3 * total * sizeof(unsigned));
+  L.sover.alloc(2 * total * sizeof(unsigned));
   L.sinq.alloc(2 * words * sizeof(unsigned));
   L.scnt.alloc((size_t)nf * 4 * sizeof(unsigned));
   L.ctr.alloc(kCtrN * sizeof(unsigned long long));
-  if (!L.sR.p || !L.sfln.p || !L.spend.p || !L.sclaim.p || !L.slist.p ||
-      !L.sover.p ||
-      !L.sinq.p || !L.scnt.p || !L.ctr.p)
+  if (!L.sR.p || !L.sfln.p || !L.spend.p || !L.slist.p || !L.sover.p || !L.sinq.p || !L.scnt.p || !L.ctr.p)
     return "device allocation failed for the solver scratch";
   size_t base = 0, wbase = 0;
   bool windowed = false;
@@ -489,14 +486,16 @@ std::string Engine::solve_level(SolveLane& L, const std::vector<std::pair<int, i
     const DevRegionStore& D = reg_[kTf[tf].reg];
     hf[i] = field_view(s, tf);
     hf[i].R = L.sR.as<double4>() + base;
-    // the state is in the records while a solve runs: its staging takes T and G
+    // the state is in the records while a solve runs: its staging takes T and G,
+    // the claims the final gradient, which is written after it
     hf[i].Tn = hf[i].T;
     hf[i].Gn = hf[i].G;
+    static_assert(sizeof(ulonglong2) == sizeof(double2), "a claim takes a gradient's place");
+    hf[i].claim = reinterpret_cast<ulonglong2*>(hf[i].Gout);
     hf[i].fln = L.sfln.as<uint8_t>() + base;
     hf[i].pend = L.spend.as<double>() + base;
-    hf[i].claim = L.sclaim.as<ulonglong2>() + base;
     hf[i].list_in = L.slist.as<unsigned>() + base;
-    hf[i].over = L.sover.as<unsigned>() + 3 * base;
+    hf[i].over = L.sover.as<unsigned>() + 2 * base;
     hf[i].inq = L.sinq.as<unsigned>() + wbase;
     hf[i].wait = L.sinq.as<unsigned>() + words + wbase;
     if (e64_tiles(hf[i]) > e64_tiles_max()) return "region too large for the eikonal solver";

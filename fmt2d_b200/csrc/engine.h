@@ -145,7 +145,7 @@ struct SolveLane {
   cudaStream_t st = nullptr;
   cudaEvent_t done = nullptr;
   DevBuf fields, up, step, sx, sz, seeds, which, hw, hwpre, ctr;
-  DevBuf sR, sfln, spend, sclaim, slist, sover, sinq, scnt;
+  DevBuf sR, sfln, spend, slist, sover, sinq, scnt;
   SolveStats stats;
   bool not_converged = false;
   // pinned staging of the lane's small host <-> device copies (descriptors,
@@ -156,7 +156,7 @@ struct SolveLane {
   size_t pin_cap = 0, pin_used = 0;
   void free_all() {
     for (DevBuf* b : {&fields, &up, &step, &sx, &sz, &seeds, &which, &hw, &hwpre, &ctr, &sR, &sfln,
-                      &spend, &sclaim, &slist, &sover, &sinq, &scnt})
+                      &spend, &slist, &sover, &sinq, &scnt})
       b->free_();
     if (pin) cudaFreeHost(pin);
     pin = nullptr;
