@@ -780,6 +780,7 @@ std::string Lsqr::set_param_grid(int nx, int nz, const int* idx, int nvp, int if
   // a new parameter grid: smoothing matrices built for another no longer apply
   for (bool& h : have_sm_) h = false;
   sm_np_ = -1;
+  have_geom_ = false;
   nvp_ = nvp;
   if_start_ = nvp;
   if_n_ = if_n;
@@ -844,6 +845,7 @@ std::string Lsqr::set_matrix(int ndata, int nparm, const int* row_ptr, const int
     if (row_ptr[i + 1] < row_ptr[i]) return "row pointer not monotone";
   if (nnz > 0 && (!col || !val)) return "null column or value array";
   cudaSetDevice(device_);
+  have_matrix_ = false;   // until all of it is there
   nd_ = ndata;
   np_ = nparm;
   nnz_ = nnz;
@@ -859,7 +861,9 @@ std::string Lsqr::set_matrix(int ndata, int nparm, const int* row_ptr, const int
   k_csr_rebase<<<grid_, kLsThreads, 0, st_>>>(rp_.as<int>(), ndata + 1, col_.as<int>(), nnz, base,
                                               nparm);
   LCK(cudaGetLastError());
-  return build_csc();
+  std::string e = build_csc();
+  have_matrix_ = e.empty();
+  return e;
 }
 
 std::string Lsqr::build_csc() {
@@ -933,7 +937,7 @@ std::string Lsqr::build_tasks() {
 }
 
 std::string Lsqr::spmv(int transpose, const double* x, double* y) {
-  if (!rp_.p) return "no matrix set";
+  if (!have_matrix_) return "no matrix set";
   cudaSetDevice(device_);
   const int nin = transpose ? nd_ : np_, nout = transpose ? np_ : nd_;
   x_.alloc((size_t)std::max(nin, 1) * 8);
@@ -948,7 +952,7 @@ std::string Lsqr::spmv(int transpose, const double* x, double* y) {
 }
 
 std::string Lsqr::gtg_diag(double* out) {
-  if (!rp_.p) return "no matrix set";
+  if (!have_matrix_) return "no matrix set";
   cudaSetDevice(device_);
   y_.alloc((size_t)np_ * 8);
   if (!y_.p) return "device allocation failed";
@@ -1005,7 +1009,7 @@ std::string Lsqr::set_smoothing(const Model& m, double corr_x, double corr_z, do
   cudaSetDevice(device_);
   const int np = m.n_inv_parms;
   for (bool& h : have_sm_) h = false;
-  sm_np_ = np;
+  sm_np_ = -1;
   std::vector<int> rp, col;
   std::vector<double> val;
   // R_h -> slots 0 (R_h) and 1 (R_h^T), R_v -> 2 and 3, interface R_h -> 4
@@ -1026,12 +1030,13 @@ std::string Lsqr::set_smoothing(const Model& m, double corr_x, double corr_z, do
       have_sm_[q.slot + 1] = true;
     }
   }
+  sm_np_ = np;
   return std::string();
 }
 
 std::string Lsqr::solve(const LsqrParams& p, const double* residual, const double* gtg,
                         const double* dm_sum, double* dm, LsqrOut* out) {
-  if (!rp_.p) return "no matrix set";
+  if (!have_matrix_) return "no matrix set";
   if (!have_geom_) return "no model geometry for the smoothing operator";
   if (p.smooth_type < 1 || p.smooth_type > 3) return "smooth_type must be 1, 2 or 3";
   if (p.max_iter < 1) return "max_iter must be >= 1";
@@ -1227,7 +1232,7 @@ size_t round_up(size_t n) { return (n + kNoAllocAlign - 1) / kNoAllocAlign * kNo
 
 std::string Lsqr::solve_noalloc(const LsqrParams& p, const double* residual, const double* gtg,
                                 const double* dm_sum, double* dm, LsqrOut* out) {
-  if (!rp_.p) return "no matrix set";
+  if (!have_matrix_) return "no matrix set";
   if (!have_geom_) return "no model geometry for the smoothing operator";
   if (p.smooth_type != 1) return "smooth_type must be 1 (Laplacian)";
   if (p.max_iter < 1) return "max_iter must be >= 1";

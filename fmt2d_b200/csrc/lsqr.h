@@ -63,12 +63,12 @@ struct LsqrDev {
   int if_start = 0, if_n = 0;   // inverted interface parameters [if_start, if_start+if_n)
   const uint8_t* mask = nullptr;// 1: velocity column masked (gtg < 0.01 eps_min)
   double ws_v = 0, ws_i = 0, wd_v = 0, wd_i = 0;
-  // smooth_type and, for 2 and 3, the Gaussian operators: R_h, R_v and their
-  // transposes, the interface R_h (applied as its own adjoint, as the
-  // reference does)
   // the columns in runs for a warp each (build_tasks): first column and number
   const int2* task = nullptr;
   int ntask = 0, task_log = 0;
+  // smooth_type and, for 2 and 3, the Gaussian operators: R_h, R_v and their
+  // transposes, the interface R_h (applied as its own adjoint, as the
+  // reference does)
   int stype = 1;
   SpRows rh, rht, rv, rvt, ri;
   const double* residual = nullptr;
@@ -153,6 +153,7 @@ class Lsqr {
   double last_ms_ = 0;
   int last_launches_ = 0;
   bool have_geom_ = false;
+  bool have_matrix_ = false; // G is complete (a set that failed leaves none)
 };
 
 }  // namespace fmt2d
