@@ -228,9 +228,9 @@ __device__ __forceinline__ double rows_dot(const int* __restrict__ rp,
 }
 
 // log2 of the rows a warp takes: as many as keep every warp busy.  The layout
-// of smooth_type 3, the inversion's usual one, keeps a warp a row and the order
-// of every sum (-1): the line search's rays are traced in its solution, and a
-// ray can turn on the last bit.
+// of smooth_type 3 keeps a warp a row and the order of every sum (-1): a line
+// search's rays are traced in its solution, and a ray can turn on the last bit
+// (an iteration's RMS moved by 1.5e-4 with another order).
 __host__ __device__ inline int rows_log(int n, int nwarp) {
   int lc = 0;
   while (lc < 5 && (n >> (lc + 1)) >= nwarp) ++lc;

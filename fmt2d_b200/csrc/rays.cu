@@ -1,6 +1,6 @@
-// Ray backtrace, water-leg entry search and Frechet rows on the device, one
-// thread per pick, FP64 with the reference's expression order (this file is
-// compiled without FMA contraction, like the eikonal stencil).
+// Ray backtrace, water-leg entry search and Frechet rows on the device, a lane
+// per pick, FP64 with the reference's expression order (this file is compiled
+// without FMA contraction, like the eikonal stencil).
 //
 //   trace_ray_from_receiver2d   src/rays2d.f90:7-153
 //   trace_ray_section2d         src/rays2d.f90:157-720 (Heun steps along -grad T

@@ -1,4 +1,5 @@
-// Device ray backtrace and Frechet rows (one thread per pick, FP64).
+// Device ray backtrace and Frechet rows (a lane per pick, whole warps stepping
+// together, FP64).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>

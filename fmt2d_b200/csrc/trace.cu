@@ -1,8 +1,9 @@
 // Host side of the ray backtrace and Frechet rows: device tables of the
-// model, the two tracing passes (count, then write) and the assembly of the
-// contributions into CSR rows (read_frechet_data2d's layout: one row per pick,
-// columns ascending, entries with |value| <= 1e-30 dropped as
-// compute_frechet_for_ray2d does, src/inversion2d.f90:4761-4768).
+// model, the trace (its entries go into a pool of chunks; a second trace where
+// the pool was too small) and the assembly of the entries into CSR rows
+// (read_frechet_data2d's layout: one row per pick, columns ascending, entries
+// with |value| <= 1e-30 dropped as compute_frechet_for_ray2d does,
+// src/inversion2d.f90:4761-4768).
 #include "engine.h"
 #include "rays.cuh"
 #include <cub/device/device_radix_sort.cuh>
