@@ -1281,7 +1281,7 @@ std::string Engine::misfit_gradient(const int* src, const int* phase, const doub
   constexpr size_t kPerSlot = sizeof(AdjLink) + sizeof(AdjNode) + 2 * sizeof(unsigned) + 3 * sizeof(double) +
                               2 * sizeof(unsigned) + 2 * sizeof(unsigned) +
                               4 * sizeof(AdjRead);
-  const CallMem mem(pool_.get(), stream_);
+  const CallMem mem = call_mem();
   const size_t budget = mem.avail / 2;
   unsigned long long cnt_bad = 0, cnt_unl = 0, cnt_left = 0, cnt_reach = 0, cnt_fields = 0;
   unsigned max_rounds = 0;

@@ -204,7 +204,6 @@ double seafloor_at(const Model& m, double px) {
 
 Engine::Engine(int device) : device_(device) {
   cudaSetDevice(device_);
-  pool_ = WorkPool::of(device_);
   cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
   cudaEventCreateWithFlags(&ev_start_, cudaEventDisableTiming);
   for (SolveLane& L : lanes_) {
@@ -225,6 +224,11 @@ Engine::~Engine() {
   }
   if (ev_start_) cudaEventDestroy(ev_start_);
   if (stream_) cudaStreamDestroy(stream_);
+}
+
+CallMem Engine::call_mem() {
+  if (!pool_) pool_ = WorkPool::of(device_);
+  return CallMem(pool_.get(), stream_);
 }
 
 std::string Engine::upload(const Model& m) {

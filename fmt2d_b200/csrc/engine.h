@@ -227,11 +227,12 @@ class Engine {
  private:
   std::string solve_level(SolveLane& L, const std::vector<std::pair<int, int>>& items);
   std::string upload_trace_tables();
+  CallMem call_mem();
   void ensure_sources(int nsrc);
   Fld64 field_view(int src, int tf) const;
   int device_;
   cudaStream_t stream_ = nullptr;
-  std::shared_ptr<WorkPool> pool_;
+  std::shared_ptr<WorkPool> pool_;   // from the first call that works in it
   Model m_;
   DevRegionStore reg_[7];
   DevBuf ifc_buf_[6][6];      // z, nx, nz, vel_top, vel_bot, izc

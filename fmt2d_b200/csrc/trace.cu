@@ -193,7 +193,7 @@ std::string Engine::trace(const int* src, const int* phase, const double* rx, co
     // rays that count their entries are traced again into one of the right size
     // (sort keys and values; the rays' entries, which the sort's second buffers
     // take the place of, their chunks' owners and counter)
-    const CallMem mem = rows ? CallMem(pool_.get(), stream_) : CallMem();
+    const CallMem mem = rows ? call_mem() : CallMem();
     struct RowSpace {
       CallBuf keys, vals, ids, pvals, owner, used;
       explicit RowSpace(const CallMem& m) : keys(m), vals(m), ids(m), pvals(m), owner(m), used(m) {}
