@@ -113,9 +113,9 @@ struct SolvePlan {
 //
 // What bounds it: a step's chain of instructions (a warp runs each phase once
 // or twice a step, at about 8 cycles an instruction) times the steps of a
-// field.  2001x401, Pg+PmP, 30 sources: 16 us a step (51 us with a thread per
-// node and three arrays), 0.21 s a forward (0.72 s).  384 threads: 256 give
-// 0.23 s (too few warps for a front of 300 nodes), 512 give 0.26 s (128
+// field.  2001x401, Pg+PmP, 30 sources: 15 us a step (51 us with a thread per
+// node and three arrays), 0.193 s a forward (0.72 s).  384 threads: 256 give
+// 0.202 s (too few warps for a front of 300 nodes), 512 give 0.229 s (128
 // registers, spills).  A cluster of blocks per field was tried and was slower
 // where it was compared, with an earlier form of the evaluation (1 source:
 // 0.18 s with 8 blocks per field against 0.15 s now with one): a cluster
